@@ -97,6 +97,10 @@ int pd_maxpool2_bwd_colsum(const void* x_pad, const void* dy_pad, int N, int C, 
 int pd_colsum_finish(const float* partial, int rows, int C, float* out, int accumulate, void* stream);
 int pd_dropout_fwd(const void* x, void* y, uint8_t* mask, int64_t n, float p, uint64_t seed,
                    uint64_t offset, int dtype, void* stream);
+/* The same with a stream position in device memory: element i draws number offset + *position + i (position may be
+ * null).  A launch recorded in a CUDA graph draws new numbers at every replay if the graph advances *position.    */
+int pd_dropout_fwd_at(const void* x, void* y, uint8_t* mask, int64_t n, float p, uint64_t seed,
+                      uint64_t offset, const int64_t* position, int dtype, void* stream);
 int pd_dropout_bwd(const void* dy, const uint8_t* mask, void* dx, int64_t n, float p, int dtype,
                    void* stream);
 /* y = a + b: residual adds of the ResNet-50 / GNMT stage files.                             */

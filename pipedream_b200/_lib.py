@@ -44,6 +44,7 @@ SIGNATURES = {
     "pd_maxpool2_bwd_colsum": (I, [P, P, I, I, I, I, P, I, I, P, L, P, P]),
     "pd_colsum_finish": (I, [P, I, I, P, I, P]),
     "pd_dropout_fwd": (I, [P, P, P, L, F, U64, U64, I, P]),
+    "pd_dropout_fwd_at": (I, [P, P, P, L, F, U64, U64, P, I, P]),
     "pd_dropout_bwd": (I, [P, P, P, L, F, I, P]),
     "pd_add": (I, [P, P, P, L, I, P]),
     "pd_layernorm_workspace_bytes": (L, [L, I]),

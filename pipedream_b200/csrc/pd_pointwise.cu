@@ -297,7 +297,8 @@ __device__ __forceinline__ uint32_t mix32(uint64_t k) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 dropout_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, uint8_t* __restrict__ mask, int64_t n,
-                   float p, uint64_t seed, uint64_t offset) {
+                   float p, uint64_t seed, uint64_t offset, const int64_t* __restrict__ position) {
+  if (position != nullptr) offset += (uint64_t)*position;
   const float scale = 1.f / (1.f - p);
   const uint32_t thresh = (uint32_t)((double)p * 4294967296.0 > 4294967295.0 ? 4294967295.0
                                                                             : (double)p * 4294967296.0);
@@ -976,16 +977,21 @@ PD_EXPORT int pd_maxpool2_bwd(const void* x, const void* dy, int N, int C, int H
   return PD_OK;
 }
 
-PD_EXPORT int pd_dropout_fwd(const void* x, void* y, uint8_t* mask, int64_t n, float p,
-                             uint64_t seed, uint64_t offset, int dtype, void* stream) {
+PD_EXPORT int pd_dropout_fwd_at(const void* x, void* y, uint8_t* mask, int64_t n, float p, uint64_t seed,
+                                uint64_t offset, const int64_t* position, int dtype, void* stream) {
   int rc = pd_check_device();
   if (rc != PD_OK) return rc;
   PD_REQUIRE(x && y && mask && n >= 0 && p >= 0.f && p < 1.f, "pd_dropout_fwd: bad arguments");
   if (n == 0) return PD_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  PD_DISPATCH_T(dtype, dropout_fwd_kernel<T><<<grid_cap((n + kThreads - 1) / kThreads), kThreads, 0, s>>>((const T*)x, (T*)y, mask, n, p, seed, offset);)
+  PD_DISPATCH_T(dtype, dropout_fwd_kernel<T><<<grid_cap((n + kThreads - 1) / kThreads), kThreads, 0, s>>>((const T*)x, (T*)y, mask, n, p, seed, offset, position);)
   PD_LAUNCH_CHECK("dropout_fwd_kernel");
   return PD_OK;
+}
+
+PD_EXPORT int pd_dropout_fwd(const void* x, void* y, uint8_t* mask, int64_t n, float p,
+                             uint64_t seed, uint64_t offset, int dtype, void* stream) {
+  return pd_dropout_fwd_at(x, y, mask, n, p, seed, offset, nullptr, dtype, stream);
 }
 
 PD_EXPORT int pd_dropout_bwd(const void* dy, const uint8_t* mask, void* dx, int64_t n, float p,

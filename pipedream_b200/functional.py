@@ -185,14 +185,20 @@ def relu_bwd(dy, y, out=None):
 
 
 _WS = {}
+# while a pass is being recorded (stage_graphs): the workspaces its launches keep, since recordings of two stages may
+# be replayed on different streams at the same time
+capture_workspaces = None
 
 
 def _workspace(device, nbytes):
     key = (device.index, _stream().value)
-    ws = _WS.get(key)
+    table = _WS
+    if capture_workspaces is not None and torch.cuda.is_current_stream_capturing():
+        table = capture_workspaces
+    ws = table.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _WS[key] = ws
+        table[key] = ws
     return ws
 
 
@@ -251,10 +257,12 @@ def colsum_finish(partial_rows, colsum, accumulate):
     call("pd_colsum_finish", _p(partial), rows, colsum.numel(), _p(colsum), int(accumulate), _stream())
 
 
-def dropout_fwd(x, p, seed, offset):
+def dropout_fwd(x, p, seed, offset, position=None):
+    """position: device address of an int64 that is added to `offset` when the kernel runs (a recorded launch)."""
     y = torch.empty_like(x)
     mask = torch.empty(x.shape, dtype=torch.uint8, device=x.device)
-    call("pd_dropout_fwd", _p(x), _p(y), _p(mask), x.numel(), float(p), int(seed), int(offset), dt(x), _stream())
+    call("pd_dropout_fwd_at", _p(x), _p(y), _p(mask), x.numel(), float(p), int(seed), int(offset), position, dt(x),
+         _stream())
     return y, mask
 
 

@@ -589,16 +589,16 @@ class NativeMaxPool2d(nn.Module):
 
 class _DropoutFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, p, seed, offset):
+    def forward(ctx, x, p, seed, offset, position):
         xc = x if x.is_contiguous() else x.contiguous()
-        y, mask = pf.dropout_fwd(xc, p, seed, offset)
+        y, mask = pf.dropout_fwd(xc, p, seed, offset, position)
         ctx.mask, ctx.p = mask, p
         return y
 
     @staticmethod
     def backward(ctx, dy):
         dyc = dy if dy.is_contiguous() else dy.contiguous()
-        return pf.dropout_bwd(dyc, ctx.mask, ctx.p), None, None, None
+        return pf.dropout_bwd(dyc, ctx.mask, ctx.p), None, None, None, None
 
 
 class NativeDropout(nn.Module):
@@ -607,13 +607,16 @@ class NativeDropout(nn.Module):
         self.p = float(p)
         self.seed = next(_SEED_COUNTER) * 7919 + torch.initial_seed() % (1 << 31)
         self.offset = 0
+        self._pd_recorded = None       # while a pass is recorded: (positions on the device, index, offset they stand for)
 
     def forward(self, x):
         if not self.training or self.p == 0.0:
             return x
-        off = self.offset
+        off, rec = self.offset, self._pd_recorded
         self.offset += x.numel()
-        return _DropoutFn.apply(x, self.p, self.seed, off)
+        if rec is None:
+            return _DropoutFn.apply(x, self.p, self.seed, off, None)
+        return _DropoutFn.apply(x, self.p, self.seed, off - rec[2], rec[0].data_ptr() + 8 * rec[1])
 
 
 # --------------------------------------------------------------------------- #
@@ -1236,6 +1239,7 @@ def nativize(module):
         graph = _Tracer().trace(module)
     except Exception:
         return module
+    module._pd_traced = True        # its forward is one straight line of operations (stage_graphs records such stages)
     mods = dict(module.named_modules())
 
     def target_mod(node):
@@ -1265,6 +1269,7 @@ def nativize(module):
     if rewritten:
         result = fx.GraphModule(module, graph)
         result.train(module.training)
+        result._pd_traced = True
         # children in the order of the original module, so that parameters() / state_dict() keep their order
         kids = result._modules
         order = [k for k in module._modules if k in kids] + [k for k in kids if k not in module._modules]

@@ -30,6 +30,7 @@ How it works is its own design:
   its flat gradient arena over NCCL instead of DistributedDataParallel.
 """
 import collections
+import contextlib
 import itertools
 import os
 import weakref
@@ -40,6 +41,7 @@ import torch.distributed as dist
 from . import communication
 from . import layers
 from . import runtime_utilities
+from . import stage_graphs
 
 IMAGE_CLASSIFICATION = "image_classification"
 TRANSLATION = "translation"
@@ -286,6 +288,9 @@ class StageRuntime:
         self.loader_iter = None
         self._feeder = None
         self._optimizer_ref = None
+        self._graphs = None            # stage_graphs.StageGraphs, made at the first pass
+        self._pass = None              # the recording the last forward pass was replayed from
+        self._output, self._output_is_static = None, False
 
         self.initialize(model, inputs_module_destinations, configuration_maps,
                         master_addr, rank, local_rank, num_ranks_in_server)
@@ -473,8 +478,22 @@ class StageRuntime:
         dtype = self.training_tensor_dtypes.get(name)
         return dtype is not None and dtype.is_floating_point
 
+    @property
+    def output(self):
+        """The criterion's input of the last forward pass.  A replayed pass leaves it in a buffer its next replay
+        overwrites, so it is copied when it is asked for."""
+        if self._output_is_static:
+            self._output, self._output_is_static = self._output.detach().clone(), False
+        return self._output
+
+    @output.setter
+    def output(self, value):
+        self._output, self._output_is_static = value, False
+
     def _start(self, num_iterations, shapes, forward_only):
         self.tensors = []
+        if self._graphs is not None:
+            self._graphs.release()
         self.gradients = {}
         self.tensor_shapes = shapes
         self.forward_only = forward_only
@@ -539,6 +558,8 @@ class StageRuntime:
         nbytes = 0
         for name in self._fwd_send:
             t = tensors[name]
+            if self._pass is not None and name in self._pass.out:
+                t = t.detach().clone()           # the next replay writes the recording's own buffer again
             self.comm_handler.send(name, t, backward=False, **ids)
             nbytes += t.element_size() * t.nelement()
         self.forward_stats.stats['send_tensors_size'] += nbytes
@@ -585,7 +606,7 @@ class StageRuntime:
             keep["_replay"] = state
             self.tensors[-1] = keep
         else:
-            self._run_forward(tensors)
+            self._forward_pass(tensors)
         if self.comm_handler is not None:
             self.send_tensors_forward()
         if "_replay" in self.tensors[-1]:
@@ -596,6 +617,17 @@ class StageRuntime:
             self.forward_stats.print_stats()
         self.forward_stats.reset_stats()
         self.forward_minibatch_id += 1
+
+    def _forward_pass(self, tensors):
+        if self._graphs is None:
+            self._graphs = stage_graphs.StageGraphs(self)
+        self._pass = None
+        if not self._graphs.usable:
+            self._run_forward(tensors)
+            return
+        self._pass = self._graphs.forward(self, tensors)
+        if self._pass is not None and self._pass.busy:
+            tensors["_pass"] = self._pass
 
     def _run_forward(self, tensors):
         self.plan.run(tensors)
@@ -643,24 +675,10 @@ class StageRuntime:
         if "_replay" in tensors:
             tensors = self._replay_forward(tensors)
 
-        roots, root_grads = [], []
-        for name in self.plan.outputs:
-            t = tensors[name]
-            if not (torch.is_tensor(t) and t.requires_grad):
-                continue
-            if name == "loss" and self.loss_scale != 1:
-                t = t * self.loss_scale
-            roots.append(t)
-            root_grads.append(self.gradients.get(name))
-        torch.autograd.backward(tuple(roots), grad_tensors=tuple(root_grads))
-
-        for name in self._bwd_send:
-            t = tensors[name]
-            g = t.grad
-            if g is None:
-                g = torch.zeros_like(t)          # an input the stage did not use
-            self.gradients[name] = g
-            t.grad = None
+        if "_pass" in tensors:
+            self._graphs.backward(self, tensors["_pass"])
+        else:
+            self._run_backward(tensors)
         if self.comm_handler is not None:
             self.send_tensors_backward()
         for name in self._bwd_recv:
@@ -671,6 +689,29 @@ class StageRuntime:
             self.backward_stats.print_stats()
         self.backward_stats.reset_stats()
         self.backward_minibatch_id += 1
+
+    def _run_backward(self, tensors):
+        roots, root_grads = [], []
+        for name in self.plan.outputs:
+            t = tensors[name]
+            if not (torch.is_tensor(t) and t.requires_grad):
+                continue
+            if name == "loss" and self.loss_scale != 1:
+                t = t * self.loss_scale
+            roots.append(t)
+            root_grads.append(self.gradients.get(name))
+        around = self._graphs.around_backward() if self._graphs is not None and self._graphs.usable \
+            else contextlib.nullcontext()
+        with around:
+            torch.autograd.backward(tuple(roots), grad_tensors=tuple(root_grads))
+
+        for name in self._bwd_send:
+            t = tensors[name]
+            g = t.grad
+            if g is None:
+                g = torch.zeros_like(t)          # an input the stage did not use
+            self.gradients[name] = g
+            t.grad = None
 
     def num_tokens(self):
         return self.tensors[-1]["target_length"][0].item()
