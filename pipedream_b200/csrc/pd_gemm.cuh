@@ -60,3 +60,5 @@ struct CUtensorMap_st;
 int pd_make_map_2d(CUtensorMap_st* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_cols,
                    int box_rows);
 int pd_gemm_launch_simt(const PdGemm& g, cudaStream_t stream);
+// K slices the fp32 back end wants for a weight gradient (k units of 64).
+int pd_gemm_simt_split(int M, int N, int num_z, int units);

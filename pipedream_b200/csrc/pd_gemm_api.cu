@@ -65,13 +65,7 @@ int grad_split(int dtype, int M, int N, int num_z, int z_per_cta, int bm, int bn
     const int sp = auto_split(ptiles, kblocks, sms / 2);
     if (pd_gemm_use_pair(M, N, num_z, z_per_cta, sp)) return sp;
   }
-  if (dtype == PD_F32) {
-    // CUDA-core tiles: two blocks per SM, the largest tile the output fills (see pd_gemm_simt_tile)
-    bm = M > 64 ? 128 : 64;
-    bn = M > 64 && N > 64 ? 128 : 64;
-    const int64_t tiles = (int64_t)num_z * ((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-    return auto_split(tiles, kblocks, 2 * sms);
-  }
+  if (dtype == PD_F32) return pd_gemm_simt_split(M, N, num_z, kblocks);
   const int64_t tiles = (int64_t)((num_z + z_per_cta - 1) / z_per_cta) * ((M + bm - 1) / bm) * ((N + bn - 1) / bn);
   return auto_split(tiles, kblocks, sms);
 }

@@ -5,16 +5,20 @@
 // Bound by the FMA pipe: 128 lanes per SM, 74 TFLOP/s at 1.965 GHz.  Every thread keeps an 8 x 8 block of outputs in
 // registers, so that one k-step is 32 packed FMAs (fma.rn.f32x2, two lanes' worth per issue slot) on four 16-byte
 // shared-memory reads; operands move from global memory to registers one chunk of 16 k ahead, and from there into the
-// other half of a double-buffered shared tile, so a chunk costs one barrier.  Three tiles share the code: a block of 256
+// other half of a double-buffered shared tile, so a chunk costs one barrier.  Four tiles share the code: a block of 256
 // threads is KG groups, and each group computes the whole BM x BN tile over its own 16 / KG of a chunk's k-steps; the
-// groups' sums are added once at the end.  That keeps the 8 x 8 register blocks for tiles a quarter the size, which is
+// groups' sums are added once at the end.  That keeps the 8 x 8 register blocks for tiles an eighth the size, which is
 // what a problem with few output tiles (a 7 x 7 feature map, a weight gradient) needs to occupy the SMs.
-// The tile with 4 x 4 outputs per thread and no double buffering that this replaced ran at 16 TFLOP/s (VGG-16, batch 8).
+// Measured: 48 to 52 TFLOP/s on 8192 x 4096 x 1024 (FMA pipe 72 % busy, shared memory 72 %), 40 to 47 on VGG-16's 3x3
+// convolutions at batch 8, 12 to 28 on ResNet-50's at batch 7; a tile with 4 x 4 outputs per thread and no double
+// buffering ran at 16 (VGG-16) and 10 (ResNet-50).
 #include "pd_gemm.cuh"
+#include <mutex>
 
 namespace {
 
-constexpr int BK = 16, kThreads = 256;
+constexpr int kThreads = 256;
+constexpr int kSplitUnit = 32;                       // K slices start at multiples of this
 
 struct SParams {
   const float* a; long long a_rows, lda; int a_major, a_vec;
@@ -44,31 +48,69 @@ __device__ __forceinline__ float2 halves(unsigned long long v) {
   return f;
 }
 
-// One operand's part of a chunk: ROWS (m or n) x 16 (k) values, as ROWS * 4 / 256 float4 per thread.
-template <int ROWS>
+// One operand's part of a chunk: ROWS (m or n) x BK (k) values, as ROWS * BK / 4 / 256 float4 per thread.  The smaller
+// tiles do few FMAs per chunk and keep their addresses in registers from chunk to chunk (KEEP); the largest has no
+// registers left for that and works them out anew, in the shadow of twice the FMAs.
+template <int ROWS, int BK, bool KEEP>
 struct Loader {
-  static constexpr int kQuads = ROWS * 4 / kThreads;
+  static constexpr int kQuads = ROWS * BK / 4 / kThreads;
   float4 v[kQuads];
+  const float* src[KEEP ? kQuads : 1];
+  const float* base;
+  long long ld, rows, first;      // first: row of the operand that row 0 (k-major) / k 0 (row-major) of the tile is
+  int limit;                      // rows (k-major) / columns (row-major) of the tile that exist
+  int have;                       // KEEP, k-major: bit q set = the row of quad q exists
 
+  __device__ __forceinline__ static int krow(int q) { return ((threadIdx.x + q * kThreads) >> 1) % ROWS; }
+  __device__ __forceinline__ static int kcol(int q) {
+    const int id = threadIdx.x + q * kThreads;
+    return (id & 1) * 4 + (id >> 1) / ROWS * 8;
+  }
+  __device__ __forceinline__ static int mrow(int q) { return (threadIdx.x + q * kThreads) / (ROWS / 4); }
+  __device__ __forceinline__ static int mcol() { return (threadIdx.x % (ROWS / 4)) * 4; }
+
+  __device__ __forceinline__ void tap(bool k_major, const float* from, long long ld_, long long rows_, long long first_,
+                                      int limit_) {
+    base = from; ld = ld_; rows = rows_; first = first_; limit = limit_;
+    if constexpr (KEEP) {
+      have = 0;
+#pragma unroll
+      for (int q = 0; q < kQuads; ++q) {
+        if (k_major) {
+          const long long gr = first + krow(q);
+          if (krow(q) < limit && gr >= 0 && gr < rows) have |= 1 << q;
+          src[q] = base + gr * ld + kcol(q);
+        } else {
+          src[q] = base + (first + mrow(q)) * ld + mcol();
+        }
+      }
+    }
+  }
   // k contiguous in memory: two neighbouring lanes read one 32-byte sector of a row; the transposed stores into
   // [k][row] (row stride ROWS + 4 floats) then hit 32 different banks.
-  __device__ __forceinline__ void load_k(const float* base, long long ld, long long rows, long long row_first, int col,
-                                         int limit, int k0, int k_end, int vec) {
+  __device__ __forceinline__ void load_k(int k0, int k_end, int vec) {
 #pragma unroll
     for (int q = 0; q < kQuads; ++q) {
-      const int id = threadIdx.x + q * kThreads;
-      const int row = (id >> 1) & (ROWS - 1), k = k0 + (id & 1) * 4 + (id >> 1) / ROWS * 8;
-      const long long gr = row_first + row;
+      const int k = k0 + kcol(q);
+      const float* s;
+      bool ok;
+      if constexpr (KEEP) {
+        s = src[q] + k0;
+        ok = (have >> q) & 1;
+      } else {
+        const long long gr = first + krow(q);
+        ok = krow(q) < limit && gr >= 0 && gr < rows;
+        s = base + gr * ld + k;
+      }
       float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (row < limit && gr >= 0 && gr < rows) {
-        const float* src = base + gr * ld + col + k;
+      if (ok) {
         if (vec && k + 4 <= k_end) {
-          f = __ldg(reinterpret_cast<const float4*>(src));
+          f = __ldg(reinterpret_cast<const float4*>(s));
         } else {
-          if (k < k_end) f.x = src[0];
-          if (k + 1 < k_end) f.y = src[1];
-          if (k + 2 < k_end) f.z = src[2];
-          if (k + 3 < k_end) f.w = src[3];
+          if (k < k_end) f.x = s[0];
+          if (k + 1 < k_end) f.y = s[1];
+          if (k + 2 < k_end) f.z = s[2];
+          if (k + 3 < k_end) f.w = s[3];
         }
       }
       v[q] = f;
@@ -77,29 +119,29 @@ struct Loader {
   __device__ __forceinline__ void store_k(float (*tile)[ROWS + 4]) const {
 #pragma unroll
     for (int q = 0; q < kQuads; ++q) {
-      const int id = threadIdx.x + q * kThreads;
-      const int row = (id >> 1) & (ROWS - 1), k = (id & 1) * 4 + (id >> 1) / ROWS * 8;
+      const int row = krow(q), k = kcol(q);
       tile[k][row] = v[q].x; tile[k + 1][row] = v[q].y; tile[k + 2][row] = v[q].z; tile[k + 3][row] = v[q].w;
     }
   }
   // rows contiguous in memory: 16-byte reads and stores along them
-  __device__ __forceinline__ void load_m(const float* base, long long ld, long long rows, long long row_first, int col,
-                                         int limit, int k0, int k_end, int vec) {
+  __device__ __forceinline__ void load_m(int k0, int k_end, int vec) {
+    const int m = mcol();
 #pragma unroll
     for (int q = 0; q < kQuads; ++q) {
-      const int id = threadIdx.x + q * kThreads;
-      const int m = (id % (ROWS / 4)) * 4, k = k0 + id / (ROWS / 4);
-      const long long gr = row_first + k;
+      const int k = k0 + mrow(q);
+      const long long gr = first + k;
+      const float* s;
+      if constexpr (KEEP) s = src[q] + (long long)k0 * ld;
+      else s = base + gr * ld + m;
       float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
       if (k < k_end && gr >= 0 && gr < rows) {
-        const float* src = base + gr * ld + col + m;
         if (vec && m + 4 <= limit) {
-          f = __ldg(reinterpret_cast<const float4*>(src));
+          f = __ldg(reinterpret_cast<const float4*>(s));
         } else {
-          if (m < limit) f.x = src[0];
-          if (m + 1 < limit) f.y = src[1];
-          if (m + 2 < limit) f.z = src[2];
-          if (m + 3 < limit) f.w = src[3];
+          if (m < limit) f.x = s[0];
+          if (m + 1 < limit) f.y = s[1];
+          if (m + 2 < limit) f.z = s[2];
+          if (m + 3 < limit) f.w = s[3];
         }
       }
       v[q] = f;
@@ -107,30 +149,25 @@ struct Loader {
   }
   __device__ __forceinline__ void store_m(float (*tile)[ROWS + 4]) const {
 #pragma unroll
-    for (int q = 0; q < kQuads; ++q) {
-      const int id = threadIdx.x + q * kThreads;
-      *reinterpret_cast<float4*>(&tile[id / (ROWS / 4)][(id % (ROWS / 4)) * 4]) = v[q];
-    }
+    for (int q = 0; q < kQuads; ++q) *reinterpret_cast<float4*>(&tile[mrow(q)][mcol()]) = v[q];
   }
 };
 
-template <int BM, int BN>
+template <int BM, int BN, int BK>
 struct Tiles {
   float a[2][BK][BM + 4];
   float b[2][BK][BN + 4];
 };
 
-template <int BM, int BN, int KG>
+template <int BM, int BN, int KG, int BK>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_simt_kernel(const __grid_constant__ SParams p) {
   static_assert(BM * BN * KG == 64 * kThreads, "8 x 8 outputs per thread");
   constexpr int kGroup = kThreads / KG;              // threads of a k-group
   constexpr int kTx = BN / 8;                        // threads across n
-  union Shared {
-    Tiles<BM, BN> t;
-    float part[KG > 1 ? kGroup * 64 : 1];
-  };
-  __shared__ __align__(16) Shared sh;
+  extern __shared__ __align__(16) unsigned char smem[];
+  Tiles<BM, BN, BK>& t = *reinterpret_cast<Tiles<BM, BN, BK>*>(smem);
+  float* part = reinterpret_cast<float*>(smem);      // after the last chunk: one group's sums
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int z = blockIdx.z / p.split_k, split = blockIdx.z % p.split_k;
   const int k_begin = split * p.k_per_split;
@@ -138,10 +175,10 @@ gemm_simt_kernel(const __grid_constant__ SParams p) {
   const int chunks = (k_end - k_begin + BK - 1) / BK;
   const int total = chunks * p.num_taps;
   const int group = threadIdx.x / kGroup, lid = threadIdx.x % kGroup;
-  // a warp covers 4 x 8 threads (32 m x 64 n of the tile): one shared-memory wavefront per operand read
+  // a warp covers 4 x 8 threads (or 8 x 4, in the narrowest tile): one shared-memory wavefront per operand read
   const int warp = lid >> 5, lane = lid & 31;
-  constexpr int kWarpsX = kTx / 8;
-  const int tx = (warp % kWarpsX) * 8 + (lane & 7), ty = (warp / kWarpsX) * 4 + (lane >> 3);
+  constexpr int kLx = kTx < 8 ? kTx : 8, kLy = 32 / kLx, kWarpsX = kTx / kLx;
+  const int tx = (warp % kWarpsX) * kLx + lane % kLx, ty = (warp / kWarpsX) * kLy + lane / kLx;
 
   unsigned long long acc[8][4];
 #pragma unroll
@@ -149,29 +186,27 @@ gemm_simt_kernel(const __grid_constant__ SParams p) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
 
-  Loader<BM> la;
-  Loader<BN> lb;
-  int tap = 0, chunk = 0;
+  Loader<BM, BK, (KG > 1)> la;
+  Loader<BN, BK, (KG > 1)> lb;
+  int tap = -1, chunk = chunks - 1;
   auto fetch = [&]() {
+    if (++chunk == chunks) {
+      chunk = 0;
+      ++tap;
+      const long long ar = (long long)p.a_row0 + p.a_tap_row[tap], br = (long long)p.b_row0 + p.b_tap_row[tap] + p.z_b_row[z];
+      const int ac = p.a_col0 + p.a_tap_col[tap], bc = p.b_col0 + p.b_tap_col[tap];
+      if (p.a_major == 0) la.tap(true, p.a + ac, p.lda, p.a_rows, ar + m0, p.M - m0);
+      else la.tap(false, p.a + ac + m0, p.lda, p.a_rows, ar, p.M - m0);
+      if (p.b_major == 0) lb.tap(true, p.b + bc, p.ldb, p.b_rows, br + n0, p.N - n0);
+      else lb.tap(false, p.b + bc + n0, p.ldb, p.b_rows, br, p.N - n0);
+    }
     const int k0 = k_begin + chunk * BK;
-    if (p.a_major == 0)
-      la.load_k(p.a, p.lda, p.a_rows, (long long)p.a_row0 + m0 + p.a_tap_row[tap], p.a_col0 + p.a_tap_col[tap], p.M - m0,
-                k0, k_end, p.a_vec);
-    else
-      la.load_m(p.a, p.lda, p.a_rows, (long long)p.a_row0 + p.a_tap_row[tap], p.a_col0 + p.a_tap_col[tap] + m0, p.M - m0,
-                k0, k_end, p.a_vec);
-    const int zr = p.z_b_row[z];
-    if (p.b_major == 0)
-      lb.load_k(p.b, p.ldb, p.b_rows, (long long)p.b_row0 + n0 + p.b_tap_row[tap] + zr, p.b_col0 + p.b_tap_col[tap],
-                p.N - n0, k0, k_end, p.b_vec);
-    else
-      lb.load_m(p.b, p.ldb, p.b_rows, (long long)p.b_row0 + p.b_tap_row[tap] + zr, p.b_col0 + p.b_tap_col[tap] + n0,
-                p.N - n0, k0, k_end, p.b_vec);
-    if (++chunk == chunks) { chunk = 0; ++tap; }
+    if (p.a_major == 0) la.load_k(k0, k_end, p.a_vec); else la.load_m(k0, k_end, p.a_vec);
+    if (p.b_major == 0) lb.load_k(k0, k_end, p.b_vec); else lb.load_m(k0, k_end, p.b_vec);
   };
   auto put = [&](int buf) {
-    if (p.a_major == 0) la.store_k(sh.t.a[buf]); else la.store_m(sh.t.a[buf]);
-    if (p.b_major == 0) lb.store_k(sh.t.b[buf]); else lb.store_m(sh.t.b[buf]);
+    if (p.a_major == 0) la.store_k(t.a[buf]); else la.store_m(t.a[buf]);
+    if (p.b_major == 0) lb.store_k(t.b[buf]); else lb.store_m(t.b[buf]);
   };
 
   fetch();
@@ -183,10 +218,10 @@ gemm_simt_kernel(const __grid_constant__ SParams p) {
 #pragma unroll
     for (int s = 0; s < BK / KG; ++s) {
       const int kk = group * (BK / KG) + s;
-      const float4 a0 = *reinterpret_cast<const float4*>(&sh.t.a[buf][kk][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&sh.t.a[buf][kk][BM / 2 + ty * 4]);
-      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&sh.t.b[buf][kk][tx * 4]);
-      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&sh.t.b[buf][kk][BN / 2 + tx * 4]);
+      const float4 a0 = *reinterpret_cast<const float4*>(&t.a[buf][kk][ty * 4]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&t.a[buf][kk][BM / 2 + ty * 4]);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&t.b[buf][kk][tx * 4]);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&t.b[buf][kk][BN / 2 + tx * 4]);
       const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -214,12 +249,12 @@ gemm_simt_kernel(const __grid_constant__ SParams p) {
     for (int g = 1; g < KG; ++g) {
       if (group == g) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i) sh.part[i * kGroup + lid] = v[i >> 3][i & 7];
+        for (int i = 0; i < 64; ++i) part[i * kGroup + lid] = v[i >> 3][i & 7];
       }
       __syncthreads();
       if (group == 0) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i) v[i >> 3][i & 7] += sh.part[i * kGroup + lid];
+        for (int i = 0; i < 64; ++i) v[i >> 3][i & 7] += part[i * kGroup + lid];
       }
       __syncthreads();
     }
@@ -269,6 +304,102 @@ gemm_simt_kernel(const __grid_constant__ SParams p) {
   }
 }
 
+// ---- a handful of rows: Linear forward and data gradient at a batch of at most eight --------------------------------
+// The weights are the whole cost (411 MB for the first Linear layer of VGG-16, 64 us at the measured copy rate) and a
+// 64-row tile would waste 7/8 of its FMAs and, with one block per 64 columns, most of the chip.  The weights are read
+// once, straight into registers; the few rows of `a` come through the L1 cache.
+constexpr int kFewRows = 8;
+
+__device__ __forceinline__ float few_epilogue(const SParams& p, float x, int m, int n) {
+  if (p.bias) x += p.bias[n];
+  if (p.relu) x = fmaxf(x, 0.f);
+  if (p.relu_aux && !(p.relu_aux[(long long)m * p.ld_aux + n] > 0.f)) x = 0.f;
+  return x;
+}
+
+// out[m, n] = sum_k a[m, k] b[n, k]: a block owns eight rows of b, four per half of its warps; the four warps of a half
+// take every fourth 128-wide piece of k.  4096 x 25088 weights: 1293 us with the tiles above.
+__global__ void __launch_bounds__(kThreads, 2)
+few_rows_nt_kernel(const __grid_constant__ SParams p) {
+  constexpr int R = 4, S = 4;
+  __shared__ float part[kThreads / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n0 = (blockIdx.x * 2 + warp / S) * R;
+  float acc[kFewRows][R];
+#pragma unroll
+  for (int m = 0; m < kFewRows; ++m)
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[m][r] = 0.f;
+  const float* b[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) b[r] = p.b + (long long)min(n0 + r, p.N - 1) * p.ldb;
+#pragma unroll 2
+  for (int k = ((warp % S) * 32 + lane) * 4; k < p.K; k += S * 128) {
+    float4 w[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) w[r] = __ldcs(reinterpret_cast<const float4*>(b[r] + k));
+#pragma unroll
+    for (int m = 0; m < kFewRows; ++m) {
+      const float4 x = __ldg(reinterpret_cast<const float4*>(p.a + (long long)min(m, p.M - 1) * p.lda + k));
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        acc[m][r] = fmaf(x.w, w[r].w, fmaf(x.z, w[r].z, fmaf(x.y, w[r].y, fmaf(x.x, w[r].x, acc[m][r]))));
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < kFewRows; ++m)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float x = pd_warp_sum(acc[m][r]);
+      if (lane == m * R + r) part[warp][lane] = x;
+    }
+  __syncthreads();
+  if (warp % S == 0) {
+    const int m = lane / R, n = n0 + lane % R;
+    if (m < p.M && n < p.N) {
+      float x = part[warp][lane];
+#pragma unroll
+      for (int w = 1; w < S; ++w) x += part[warp + w][lane];
+      p.out[(long long)m * p.ldo + n] = few_epilogue(p, x, m, n);
+    }
+  }
+}
+
+// out[m, n] = sum_k a[m, k] b[k, n]: a block owns 32 columns, its 16 warps a sixteenth of k each.
+__global__ void __launch_bounds__(512)
+few_rows_nn_kernel(const __grid_constant__ SParams p) {
+  constexpr int kWarps = 16;
+  __shared__ float part[kWarps][kFewRows][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = blockIdx.x * 32 + lane;
+  const int per = ((p.K + kWarps - 1) / kWarps + 3) / 4 * 4;
+  const int k_begin = warp * per, k_end = min(p.K, k_begin + per);
+  float acc[kFewRows];
+#pragma unroll
+  for (int m = 0; m < kFewRows; ++m) acc[m] = 0.f;
+  const float* b = p.b + min(n, p.N - 1);
+#pragma unroll 4
+  for (int k = k_begin; k < k_end; k += 4) {         // K is a multiple of four
+    float w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = __ldcs(b + (long long)(k + j) * p.ldb);
+#pragma unroll
+    for (int m = 0; m < kFewRows; ++m) {
+      const float4 x = __ldg(reinterpret_cast<const float4*>(p.a + (long long)min(m, p.M - 1) * p.lda + k));
+      acc[m] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], acc[m]))));
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < kFewRows; ++m) part[warp][m][lane] = acc[m];
+  __syncthreads();
+  if (warp < p.M && warp < kFewRows && n < p.N) {
+    float x = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) x += part[w][warp][lane];
+    p.out[(long long)warp * p.ldo + n] = few_epilogue(p, x, warp, n);
+  }
+}
+
 // 16-byte reads need every row start on a 16-byte boundary, tap and origin columns included.
 int vectorised(const void* base, long long ld, int col0, const int* tap_col, int taps) {
   if (((uintptr_t)base & 15) || (ld & 3) || (col0 & 3)) return 0;
@@ -279,15 +410,60 @@ int vectorised(const void* base, long long ld, int col0, const int* tap_col, int
 
 }  // namespace
 
-// Tile of an fp32 problem with `outer` independent outputs (z x K slices): the largest that still gives (nearly) every
-// SM its two blocks; below that the tile that spreads the work over the most SMs (a block of the small tile takes a
-// quarter of the large one's time).  Returns the tile's BM in *bm and BN in *bn.
-static void pd_gemm_simt_tile(int M, int N, long long outer, int* bm, int* bn) {
-  const long long full = 2ll * pd_num_sms() * 7 / 8;
-  const auto tiles = [&](int tm, int tn) { return (long long)((M + tm - 1) / tm) * ((N + tn - 1) / tn) * outer; };
-  if (N > 64 && M > 64 && tiles(128, 128) >= full) { *bm = 128; *bn = 128; return; }
-  if (M > 64 && tiles(128, 64) >= full) { *bm = 128; *bn = 64; return; }
-  *bm = 64; *bn = 64;
+namespace {
+
+struct SimtTile {
+  int bm, bn;
+  double rate;                  // TFLOP/s of a problem that fills the chip with it (measured)
+  int smem;
+  void (*kernel)(SParams);
+};
+template <int BM, int BN, int KG, int BK>
+SimtTile simt_tile(double rate) {
+  const int tiles = (int)sizeof(Tiles<BM, BN, BK>), part = KG > 1 ? BM * BN * 4 : 0;
+  return {BM, BN, rate, tiles > part ? tiles : part, gemm_simt_kernel<BM, BN, KG, BK>};
+}
+const SimtTile kTiles[4] = {simt_tile<128, 128, 1, 16>(49.), simt_tile<128, 64, 2, 16>(40.),
+                            simt_tile<64, 64, 4, 32>(37.), simt_tile<64, 32, 8, 32>(28.)};
+std::mutex g_simt_mu;
+bool g_simt_ready[64];
+
+// Estimated time in us of `blocks` blocks of a tile with k steps each: two of them share an SM; one alone gets three
+// quarters of the SM's rate out of it; filling the pipeline and the epilogue cost about 3.6 us per block of an SM whatever
+// the tile.  (Within a tenth of the measured times of ResNet-50's layers at batch 7, K from 64 to 4608.)  The smaller
+// tiles lose to the larger ones on rate and win where the larger ones leave SMs idle in the last, often only, round.
+double tile_time(const SimtTile& t, long long blocks, double k) {
+  const long long sms = pd_num_sms(), n = (blocks + sms - 1) / sms;
+  const double per_k = 2. * t.bm * t.bn / (t.rate * 1e6 / sms) * ((double)(n - n % 2) + (double)(n % 2) / 0.75);
+  return per_k * k + 3.6 * n;
+}
+const SimtTile& pick_tile(int M, int N, long long outer, double k, double* time = nullptr) {
+  const SimtTile* best = nullptr;
+  double best_time = 0.;
+  for (const SimtTile& t : kTiles) {
+    const double e = tile_time(t, (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn) * outer, k);
+    if (!best || e < best_time) { best = &t; best_time = e; }
+  }
+  if (time) *time = best_time;
+  return *best;
+}
+
+}  // namespace
+
+// K slices for a weight gradient of num_z outputs [M, N] over k units of 64: the count that takes the least time with the
+// tile picked for it.  Slices of one output add up at the same addresses, which takes about 0.3 us a slice.
+int pd_gemm_simt_split(int M, int N, int num_z, int units) {
+  int best = 1;
+  double best_time = 1e300;
+  for (int s = 1; s <= 128 && s <= units; ++s) {
+    const int per = (units + s - 1) / s, used = (units + per - 1) / per;
+    if (used != s) continue;
+    double time;
+    pick_tile(M, N, (long long)num_z * used, 64. * per, &time);
+    if (used > 1) time += 2. + 0.3 * used;
+    if (time < best_time) { best_time = time; best = used; }
+  }
+  return best;
 }
 
 int pd_gemm_launch_simt(const PdGemm& g, cudaStream_t stream) {
@@ -310,21 +486,37 @@ int pd_gemm_launch_simt(const PdGemm& g, cudaStream_t stream) {
   p.a_vec = vectorised(g.a, g.lda, g.a_col0, g.a_tap_col, g.num_taps);
   p.b_vec = vectorised(g.b, g.ldb, g.b_col0, g.b_tap_col, g.num_taps);
   p.z_out_col = g.z_out_col;
-  int kblocks = (g.K + BK - 1) / BK;
+  const int kblocks = (g.K + kSplitUnit - 1) / kSplitUnit;
   int split = g.split_k > kblocks ? kblocks : g.split_k;
-  int per = (kblocks + split - 1) / split;
+  const int per = (kblocks + split - 1) / split;
   split = (kblocks + per - 1) / per;
-  p.split_k = split; p.k_per_split = per * BK;
+  p.split_k = split; p.k_per_split = per * kSplitUnit;
   p.out = (float*)g.out; p.ldo = g.ldo; p.atomic = g.atomic;
   p.bias = (const float*)g.bias; p.relu = g.relu; p.pad_hp = g.pad_hp; p.pad_wp = g.pad_wp;
   p.relu_aux = (const float*)g.relu_aux; p.ld_aux = g.ld_aux;
-  int bm, bn;
-  pd_gemm_simt_tile(g.M, g.N, (long long)g.num_z * split, &bm, &bn);
-  dim3 grid((g.M + bm - 1) / bm, (g.N + bn - 1) / bn, g.num_z * split);
+  if (p.M <= kFewRows && !p.a_major && p.num_taps == 1 && g.num_z == 1 && split == 1 && !p.atomic && p.pad_wp == 0 &&
+      p.a_row0 == 0 && p.b_row0 == 0 && p.a_col0 == 0 && p.b_col0 == 0 && p.a_tap_row[0] == 0 && p.b_tap_row[0] == 0 &&
+      p.a_tap_col[0] == 0 && p.b_tap_col[0] == 0 && p.z_b_row[0] == 0 && p.a_vec && p.b_vec && p.K % 4 == 0 &&
+      p.a_rows >= p.M && p.b_rows >= (p.b_major ? p.K : p.N)) {
+    if (p.b_major) few_rows_nn_kernel<<<(p.N + 31) / 32, 512, 0, stream>>>(p);
+    else few_rows_nt_kernel<<<(p.N + 7) / 8, kThreads, 0, stream>>>(p);
+    PD_LAUNCH_CHECK("few_rows_kernel");
+    return PD_OK;
+  }
+  const SimtTile& t = pick_tile(g.M, g.N, (long long)g.num_z * split, (double)p.num_taps * (p.k_per_split < p.K ? p.k_per_split : p.K));
+  {
+    int dev = 0;
+    PD_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_simt_mu);
+    if (dev >= 0 && dev < 64 && !g_simt_ready[dev]) {
+      for (const SimtTile& k : kTiles)
+        PD_CUDA(cudaFuncSetAttribute((const void*)k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
+      g_simt_ready[dev] = true;
+    }
+  }
+  dim3 grid((g.M + t.bm - 1) / t.bm, (g.N + t.bn - 1) / t.bn, g.num_z * split);
   PD_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "simt gemm: grid too large");
-  if (bm == 128 && bn == 128) gemm_simt_kernel<128, 128, 1><<<grid, kThreads, 0, stream>>>(p);
-  else if (bm == 128) gemm_simt_kernel<128, 64, 2><<<grid, kThreads, 0, stream>>>(p);
-  else gemm_simt_kernel<64, 64, 4><<<grid, kThreads, 0, stream>>>(p);
+  t.kernel<<<grid, kThreads, t.smem, stream>>>(p);
   PD_LAUNCH_CHECK("gemm_simt_kernel");
   return PD_OK;
 }

@@ -23,7 +23,7 @@ def _check(got, a, b, k):
 # 64x64 tile; 128x64 (many rows, narrow); 128x128; odd leading dimensions; K below, at and past a chunk of 16
 @pytest.mark.parametrize("M,N,K,odd", [(1, 8, 1, False), (63, 65, 15, True), (64, 64, 16, False), (130, 129, 17, False),
                                        (40001, 64, 33, False), (40001, 61, 9, True), (5003, 1030, 48, False),
-                                       (5003, 1029, 31, True), (7, 1000, 2048, False)])
+                                       (5003, 1029, 31, True), (7, 1000, 2048, False), (8, 34, 132, False), (1, 66, 4, False), (8, 4096, 516, False)])
 def test_tiles(M, N, K, odd):
     ld = lambda n: n + 3 if odd else (n + 3) // 4 * 4
     a, b = _mat(M, K, ld(K), 1), _mat(N, K, ld(K), 2)
