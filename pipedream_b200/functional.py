@@ -122,6 +122,22 @@ def padded_of(view):
     return view.as_strided((N, Hp, Wp, C), (Hp * Wp * C, Wp * C, C, 1), off)
 
 
+def copy_of(t):
+    """A copy of t that keeps the padded layout where t has it: one dense copy here, and nothing to pack later."""
+    pad = padded_of(t) if t.is_cuda and not t.is_contiguous() else None
+    return nchw_view(pad.clone(), *t.shape) if pad is not None else t.clone()
+
+
+def copy_into(dst, src):
+    """dst.copy_(src); two padded buffers are copied whole (their borders are zero), without the walk over strides."""
+    if dst.is_cuda and src.is_cuda and dst.dtype == src.dtype and dst.shape == src.shape and not src.is_contiguous():
+        a, b = padded_of(dst), padded_of(src)
+        if a is not None and b is not None:
+            a.copy_(b)
+            return
+    dst.copy_(src)
+
+
 def pack_pnhwc(x, dtype=None):
     """Any-stride [N,C,H,W] tensor -> new padded-NHWC buffer (zero border)."""
     _cuda(x)

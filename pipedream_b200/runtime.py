@@ -39,6 +39,7 @@ import torch
 import torch.distributed as dist
 
 from . import communication
+from . import functional as pf
 from . import layers
 from . import runtime_utilities
 from . import stage_graphs
@@ -559,7 +560,7 @@ class StageRuntime:
         for name in self._fwd_send:
             t = tensors[name]
             if self._pass is not None and name in self._pass.out:
-                t = t.detach().clone()           # the next replay writes the recording's own buffer again
+                t = pf.copy_of(t.detach())      # the next replay writes the recording's own buffer again
             self.comm_handler.send(name, t, backward=False, **ids)
             nbytes += t.element_size() * t.nelement()
         self.forward_stats.stats['send_tensors_size'] += nbytes

@@ -316,7 +316,7 @@ class StageGraphs:
     def _replay_forward(self, rt, p, opt, tensors, fresh):
         p.last_used = self.minibatches
         for n, s in p.data.items():
-            s.copy_(tensors[n])
+            pf.copy_into(s, tensors[n])
         if opt is not None:
             self._load_shadow(opt)
         if self.dropouts:
@@ -367,10 +367,11 @@ class StageGraphs:
             g = rt.gradients.get(n)
             if g is not None:
                 s = p.grad_in.get(n)
-                if s is None or s.shape != g.shape or s.dtype != g.dtype:
-                    s = p.grad_in[n] = torch.empty(g.shape, dtype=g.dtype, device=self.device)
+                padded = not g.is_contiguous() and pf.padded_of(g) is not None
+                if s is None or s.shape != g.shape or s.dtype != g.dtype or padded != (not s.is_contiguous()):
+                    s = p.grad_in[n] = _static_like(g) if padded else torch.empty(g.shape, dtype=g.dtype, device=self.device)
                     p.backwards.clear()
-                s.copy_(g)
+                pf.copy_into(s, g)
                 grads[n] = s
         weights, opt = self._weights(rt)
         if opt is not None:
@@ -397,7 +398,7 @@ class StageGraphs:
             leaf = b.leaf_grads
         for n in rt._bwd_send:
             g = leaf.get(n)
-            rt.gradients[n] = g.clone() if g is not None else torch.zeros_like(p.static[n])
+            rt.gradients[n] = pf.copy_of(g) if g is not None else torch.zeros_like(p.static[n])
         p.busy = False
 
     def _roots(self, rt, p, grads):
