@@ -124,6 +124,20 @@ int pd_bn_bwd(int dtype, const void* x_pad, const void* dy_pad, const void* y_pa
               const void* gamma, const float* mean, const float* invstd, float* dgamma, float* dbeta,
               int accumulate, void* dx_pad, void* dres_pad, float* sums_ws, void* workspace,
               int64_t workspace_bytes, void* stream);
+/* The same with a mask of one bit per value (y > 0), written by the forward and read by the backward pass in y's place:
+ * pd_bn_mask_bytes bytes, 0 where a shape has none (C not 8 times a power of two up to 256); mask may be NULL.
+ * pd_bn_apply_var: pd_bn_apply from a variance, invstd = 1/sqrt(var + eps).                                        */
+int64_t pd_bn_mask_bytes(int N, int H, int W, int C);
+int pd_bn_fwd_masked(int dtype, const void* x_pad, const void* res_pad, int N, int H, int W, int C, const void* gamma,
+                     const void* beta, float eps, float momentum, int relu, float* mean, float* invstd,
+                     float* running_mean, float* running_var, void* y_pad, void* mask, void* workspace,
+                     int64_t workspace_bytes, void* stream);
+int pd_bn_apply_var(int dtype, const void* x_pad, const void* res_pad, int N, int H, int W, int C, const void* gamma,
+                    const void* beta, const float* mean, const float* var, float eps, int relu, void* y_pad, void* stream);
+int pd_bn_bwd_masked(int dtype, const void* x_pad, const void* dy_pad, const void* y_pad, const void* mask, int N, int H,
+                     int W, int C, const void* gamma, const float* mean, const float* invstd, float* dgamma, float* dbeta,
+                     int accumulate, void* dx_pad, void* dres_pad, float* sums_ws, void* workspace,
+                     int64_t workspace_bytes, void* stream);
 /* Convolution variants other than 3x3/stride 1 (resnet50/gpus=4/stage0.py:10: 7x7 stride 2; 1x1 and 3x3
  * stride 2) run as a patch matrix through pd_gemm_*: pd_im2col builds [N*Ho*Wo, Kpad] (k = (r*kw+s)*C + c)
  * from an any-stride NCHW source, pd_col2im_pnhwc gathers the patch-matrix gradient back into padded NHWC. */

@@ -57,6 +57,10 @@ SIGNATURES = {
     "pd_bn_workspace_bytes": (L, [I]),
     "pd_bn_fwd": (I, [I, P, P, I, I, I, I, P, P, F, F, I, P, P, P, P, P, P, L, P]),
     "pd_bn_apply": (I, [I, P, P, I, I, I, I, P, P, P, P, I, P, P]),
+    "pd_bn_mask_bytes": (L, [I, I, I, I]),
+    "pd_bn_fwd_masked": (I, [I, P, P, I, I, I, I, P, P, F, F, I, P, P, P, P, P, P, P, L, P]),
+    "pd_bn_apply_var": (I, [I, P, P, I, I, I, I, P, P, P, P, F, I, P, P]),
+    "pd_bn_bwd_masked": (I, [I, P, P, P, P, I, I, I, I, P, P, P, P, P, I, P, P, P, P, L, P]),
     "pd_bn_bwd": (I, [I, P, P, P, I, I, I, I, P, P, P, P, P, I, P, P, P, P, L, P]),
     "pd_im2col": (I, [P, I, L, L, L, L, I, I, I, I, I, I, I, I, I, I, I, P, I, P]),
     "pd_col2im_pnhwc": (I, [P, I, I, I, I, I, I, I, I, I, I, I, P, I, P]),

@@ -11,9 +11,10 @@
 //   backward: g = dy (zeroed where y <= 0 when the forward applied a ReLU); per-channel sum(g) and
 //             sum(g*xhat); dx = gamma*invstd*(g - sum(g)/cnt - xhat*sum(g*xhat)/cnt), border rows zero;
 //             g itself is the gradient of the residual input.
-// All kernels are HBM-bound: bf16 tensors whose channel count is a multiple of 8 with C/8 dividing 256
-// (every ResNet-50 layer) take a path with 16-byte accesses in which a thread keeps the same 8 channels
-// for the whole launch; everything else takes the generic scalar path.
+// All kernels are HBM-bound: tensors whose channel count is 8 times a power of two up to 256 (every ResNet-50
+// layer) take a path with 16-byte accesses in which a thread keeps the same 8 channels for the whole launch;
+// everything else takes the generic scalar path.  On the vector path the forward pass can leave one bit per
+// value (y > 0) for the backward pass, which then reads 1/16 of the bytes that y itself takes in its two passes.
 #include "pd_common.cuh"
 
 namespace {
@@ -27,26 +28,50 @@ __device__ __forceinline__ bool is_border(int64_t row, int Hp, int Wp) {
   return wp == 0 || wp == Wp - 1 || hp == 0 || hp == Hp - 1;
 }
 
-__device__ __forceinline__ void unpack8(const uint4& u, float* f) {
-  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 t = __bfloat1622float2(p[k]);
-    f[2 * k] = t.x;
-    f[2 * k + 1] = t.y;
-  }
-}
-
-__device__ __forceinline__ uint4 pack8(const float* f) {
+// Eight consecutive values of a channel group: 16 bytes of bf16, 32 bytes of fp32.
+template <typename T> struct Vec8;
+template <> struct Vec8<__nv_bfloat16> {
   uint4 u;
-  __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&u);
+  __device__ __forceinline__ void zero() { u = make_uint4(0u, 0u, 0u, 0u); }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p, int64_t i) { u = reinterpret_cast<const uint4*>(p)[i]; }
+  __device__ __forceinline__ void store(__nv_bfloat16* p, int64_t i) const { reinterpret_cast<uint4*>(p)[i] = u; }
+  __device__ __forceinline__ void get(float* f) const {
+    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) p[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
-  return u;
-}
+    for (int k = 0; k < 4; ++k) {
+      const float2 t = __bfloat1622float2(p[k]);
+      f[2 * k] = t.x;
+      f[2 * k + 1] = t.y;
+    }
+  }
+  __device__ __forceinline__ void set(const float* f) {
+    __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+  }
+};
+template <> struct Vec8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void zero() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ void load(const float* p, int64_t i) {
+    a = reinterpret_cast<const float4*>(p)[2 * i];
+    b = reinterpret_cast<const float4*>(p)[2 * i + 1];
+  }
+  __device__ __forceinline__ void store(float* p, int64_t i) const {
+    reinterpret_cast<float4*>(p)[2 * i] = a;
+    reinterpret_cast<float4*>(p)[2 * i + 1] = b;
+  }
+  __device__ __forceinline__ void get(float* f) const {
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+  }
+  __device__ __forceinline__ void set(const float* f) {
+    a = make_float4(f[0], f[1], f[2], f[3]);
+    b = make_float4(f[4], f[5], f[6], f[7]);
+  }
+};
 
 // ------------------------------------------------------------------------------------------------
-// generic path (fp32, or channel counts the vector path does not take)
+// generic path (channel counts the vector path does not take)
 // ------------------------------------------------------------------------------------------------
 // partial[block][0][C] = sum_r a(r,c), partial[block][1][C] = sum_r b(r,c) over the block's rows.
 //   mode 0 (forward statistics): a = x, b = x*x
@@ -89,10 +114,13 @@ bn_reduce_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __r
   }
 }
 
+// The inference path hands over running variances (eps >= 0), the training path finished 1/sqrt(var + eps) (eps < 0).
+__device__ __forceinline__ float scale_of(float v, float eps) { return eps < 0.f ? v : rsqrtf(v + eps); }
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, const float* __restrict__ mean,
-                const float* __restrict__ invstd, const T* __restrict__ gamma, const T* __restrict__ beta,
+                const float* __restrict__ invstd, float eps, const T* __restrict__ gamma, const T* __restrict__ beta,
                 int64_t rows, int C, int Hp, int Wp, int relu, T* __restrict__ y) {
   const int64_t total = rows * C;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -100,7 +128,7 @@ bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, const float*
     const int64_t r = i / C;
     float v = 0.f;
     if (!is_border(r, Hp, Wp)) {
-      v = (pd_to_float(x[i]) - mean[c]) * invstd[c] * pd_to_float(gamma[c]) + pd_to_float(beta[c]);
+      v = (pd_to_float(x[i]) - mean[c]) * scale_of(invstd[c], eps) * pd_to_float(gamma[c]) + pd_to_float(beta[c]);
       if (res != nullptr) v += pd_to_float(res[i]);
       if (relu) v = fmaxf(v, 0.f);
     }
@@ -132,16 +160,23 @@ bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* 
 
 // ------------------------------------------------------------------------------------------------
 // second level of the reductions (both paths): one block per 32 channels, 32 slices of the partials each
-// (the loop over the partials is a chain of L2 round trips: short and wide beats long and narrow)
+// (the loop over the partials is a chain of L2 round trips: short and wide beats long and narrow; 16 loads a thread
+// are in flight at a time)
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void sum_partials(const float* __restrict__ partial, int nblocks, int C, int c,
                                              float (*sh)[32][33], float& s, float& q) {
   s = q = 0.f;
   if (c < C) {
-#pragma unroll 4
-    for (int b = threadIdx.y; b < nblocks; b += 32) {
-      s += partial[((int64_t)b * 2) * C + c];
-      q += partial[((int64_t)b * 2 + 1) * C + c];
+    for (int b0 = threadIdx.y; b0 < nblocks; b0 += 32 * 8) {
+      float ps[8], pq[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int b = b0 + u * 32;
+        ps[u] = b < nblocks ? partial[((int64_t)b * 2) * C + c] : 0.f;
+        pq[u] = b < nblocks ? partial[((int64_t)b * 2 + 1) * C + c] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) { s += ps[u]; q += pq[u]; }
     }
   }
   sh[0][threadIdx.y][threadIdx.x] = s;
@@ -194,14 +229,39 @@ bn_bwd_final_kernel(const float* __restrict__ partial, int nblocks, int C, float
 }
 
 // ------------------------------------------------------------------------------------------------
-// bf16 vector path.  The matrix is read as nvec = P*C/8 16-byte vectors; G = C/8 vectors per row,
-// G a power of two <= 256, so a thread's channel group (index mod G) never changes.
+// Vector path.  The matrix is read as nvec = P*C/8 vectors of 8 values; G = C/8 vectors per row, G a power of two
+// <= 256, so a thread's channel group (index mod G) never changes.  MASK: where the forward pass applied a ReLU, what
+// says that a value passed: 0 nothing to mask, 1 the output y, 2 one byte per vector that the forward pass left.
 // ------------------------------------------------------------------------------------------------
-template <int MODE, bool MASK>
+template <typename T, int MASK>
+struct Passed {
+  Vec8<T> y;
+  unsigned char bits;
+  __device__ __forceinline__ void load(const T* yp, const unsigned char* mp, int64_t i, bool ok) {
+    if (MASK == 1) { if (ok) y.load(yp, i); else y.zero(); }
+    if (MASK == 2) bits = ok ? mp[i] : (unsigned char)0;
+  }
+  __device__ __forceinline__ void apply(float* g) const {
+    if (MASK == 1) {
+      float yf[8];
+      y.get(yf);
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (!(yf[k] > 0.f)) g[k] = 0.f;
+    }
+    if (MASK == 2) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (!((bits >> k) & 1)) g[k] = 0.f;
+    }
+  }
+};
+
+template <typename T, int MODE, int MASK>
 __global__ void __launch_bounds__(kThreads)
-bn_reduce_v8_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, const uint4* __restrict__ y,
-                    const float* __restrict__ mean, const float* __restrict__ invstd, int64_t nvec, int G, int C,
-                    float* __restrict__ partial) {
+bn_reduce_v8_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
+                    const unsigned char* __restrict__ mask, const float* __restrict__ mean,
+                    const float* __restrict__ invstd, int64_t nvec, int G, int C, float* __restrict__ partial) {
   __shared__ float sh[kThreads][17];
   const int tid = threadIdx.x;
   const int cg = tid & (G - 1);
@@ -215,35 +275,35 @@ bn_reduce_v8_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, c
   const int64_t per = (((nvec + gridDim.x - 1) / gridDim.x) + kThreads - 1) / kThreads * kThreads;
   const int64_t v0 = (int64_t)blockIdx.x * per;
   const int64_t v1 = min(nvec, v0 + per);
-  constexpr int U = MODE == 0 ? 4 : 2;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  constexpr int U = (MODE == 1 && (MASK == 1 || sizeof(T) == 4)) ? 2 : 4;
   for (int64_t base = v0 + tid; base < v1; base += (int64_t)kThreads * U) {
-    uint4 xv[U], gv[U], yv[U];
+    Vec8<T> xv[U], gv[U];
+    Passed<T, MASK> pass[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t i = base + (int64_t)u * kThreads;
       const bool ok = i < v1;
-      xv[u] = ok ? x[i] : zero;
-      if (MODE == 1) gv[u] = ok ? dy[i] : zero;
-      if (MODE == 1 && MASK) yv[u] = ok ? y[i] : zero;
+      if (ok) xv[u].load(x, i); else xv[u].zero();
+      if (MODE == 1) {
+        if (ok) gv[u].load(dy, i); else gv[u].zero();
+        pass[u].load(y, mask, i, ok);
+      }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       float xf[8];
-      unpack8(xv[u], xf);
+      xv[u].get(xf);
       if (MODE == 0) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) { a[k] += xf[k]; b[k] += xf[k] * xf[k]; }
       } else {
-        float gf[8], yf[8];
-        unpack8(gv[u], gf);
-        if (MASK) unpack8(yv[u], yf);
+        float gf[8];
+        gv[u].get(gf);
+        pass[u].apply(gf);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          float g = gf[k];
-          if (MASK && !(yf[k] > 0.f)) g = 0.f;
-          a[k] += g;
-          b[k] += g * (xf[k] - m[k]) * is[k];
+          a[k] += gf[k];
+          b[k] += gf[k] * (xf[k] - m[k]) * is[k];
         }
       }
     }
@@ -268,61 +328,69 @@ __device__ __forceinline__ bool border_of_vec(int64_t i, int gshift, int Hp, int
   return wp == 0 || wp == (unsigned)Wp - 1 || hp == 0 || hp == (unsigned)Hp - 1;
 }
 
+template <typename T>
 __global__ void __launch_bounds__(kThreads)
-bn_apply_v8_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, const float* __restrict__ mean,
-                   const float* __restrict__ invstd, const __nv_bfloat16* __restrict__ gamma,
-                   const __nv_bfloat16* __restrict__ beta, int64_t nvec, int G, int gshift, int Hp, int Wp, int relu,
-                   uint4* __restrict__ y) {
+bn_apply_v8_kernel(const T* __restrict__ x, const T* __restrict__ res, const float* __restrict__ mean,
+                   const float* __restrict__ invstd, float eps, const T* __restrict__ gamma,
+                   const T* __restrict__ beta, int64_t nvec, int G, int gshift, int Hp, int Wp, int relu,
+                   T* __restrict__ y, unsigned char* __restrict__ mask) {
   const int cg = threadIdx.x & (G - 1);
   float scale[8], shift[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int c = cg * 8 + k;
-    scale[k] = invstd[c] * __bfloat162float(gamma[c]);
-    shift[k] = __bfloat162float(beta[c]) - mean[c] * scale[k];
+    scale[k] = scale_of(invstd[c], eps) * pd_to_float(gamma[c]);
+    shift[k] = pd_to_float(beta[c]) - mean[c] * scale[k];
   }
-  constexpr int U = 4;
+  constexpr int U = sizeof(T) == 4 ? 2 : 4;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   for (int64_t base = (int64_t)blockIdx.x * kThreads + threadIdx.x; base < nvec; base += stride * U) {
-    uint4 xv[U], rv[U];
+    Vec8<T> xv[U], rv[U];
     bool ok[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t i = base + (int64_t)u * stride;
       ok[u] = i < nvec && !border_of_vec(i, gshift, Hp, Wp);
-      xv[u] = ok[u] ? x[i] : zero;
-      if (res != nullptr) rv[u] = ok[u] ? res[i] : zero;
+      if (ok[u]) xv[u].load(x, i); else xv[u].zero();
+      if (res != nullptr) { if (ok[u]) rv[u].load(res, i); else rv[u].zero(); }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t i = base + (int64_t)u * stride;
       if (i >= nvec) break;
-      uint4 out = zero;
+      Vec8<T> out;
+      out.zero();
+      unsigned int bits = 0u;
       if (ok[u]) {
         float f[8], r[8];
-        unpack8(xv[u], f);
-        if (res != nullptr) unpack8(rv[u], r);
+        xv[u].get(f);
+        if (res != nullptr) rv[u].get(r);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           float v = f[k] * scale[k] + shift[k];
           if (res != nullptr) v += r[k];
           f[k] = relu ? fmaxf(v, 0.f) : v;
         }
-        out = pack8(f);
+        out.set(f);
+        if (mask != nullptr) {
+          out.get(f);                      // as stored: what rounds to zero has not passed
+#pragma unroll
+          for (int k = 0; k < 8; ++k) bits |= f[k] > 0.f ? 1u << k : 0u;
+        }
       }
-      y[i] = out;
+      out.store(y, i);
+      if (mask != nullptr) mask[i] = (unsigned char)bits;
     }
   }
 }
 
-template <bool MASK>
+template <typename T, int MASK>
 __global__ void __launch_bounds__(kThreads)
-bn_bwd_apply_v8_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, const uint4* __restrict__ y,
-                       const float* __restrict__ mean, const float* __restrict__ invstd,
-                       const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ sums, int64_t nvec, int G,
-                       int gshift, int C, int Hp, int Wp, float inv_count, uint4* __restrict__ dx,
-                       uint4* __restrict__ dres) {
+bn_bwd_apply_v8_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
+                       const unsigned char* __restrict__ mask, const float* __restrict__ mean,
+                       const float* __restrict__ invstd, const T* __restrict__ gamma, const float* __restrict__ sums,
+                       int64_t nvec, int G, int gshift, int C, int Hp, int Wp, float inv_count, T* __restrict__ dx,
+                       T* __restrict__ dres) {
   const int cg = threadIdx.x & (G - 1);
   // dx = k1 * (g - c1 - (x - mean) * c2),  k1 = gamma*invstd, c1 = sum(g)/cnt, c2 = invstd*sum(g*xhat)/cnt
   float k1[8], c1[8], c2[8], m[8];
@@ -330,45 +398,43 @@ bn_bwd_apply_v8_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy
   for (int k = 0; k < 8; ++k) {
     const int c = cg * 8 + k;
     const float is = invstd[c];
-    k1[k] = __bfloat162float(gamma[c]) * is;
+    k1[k] = pd_to_float(gamma[c]) * is;
     c1[k] = sums[c] * inv_count;
     c2[k] = is * sums[C + c] * inv_count;
     m[k] = mean[c];
   }
-  constexpr int U = 2;
+  constexpr int U = (MASK == 1 || sizeof(T) == 4) ? 2 : 4;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   for (int64_t base = (int64_t)blockIdx.x * kThreads + threadIdx.x; base < nvec; base += stride * U) {
-    uint4 xv[U], gv[U], yv[U];
+    Vec8<T> xv[U], gv[U];
+    Passed<T, MASK> pass[U];
     bool ok[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t i = base + (int64_t)u * stride;
       ok[u] = i < nvec && !border_of_vec(i, gshift, Hp, Wp);
-      xv[u] = ok[u] ? x[i] : zero;
-      gv[u] = ok[u] ? dy[i] : zero;
-      if (MASK) yv[u] = ok[u] ? y[i] : zero;
+      if (ok[u]) { xv[u].load(x, i); gv[u].load(dy, i); } else { xv[u].zero(); gv[u].zero(); }
+      pass[u].load(y, mask, i, ok[u]);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t i = base + (int64_t)u * stride;
       if (i >= nvec) break;
-      uint4 out = zero, gout = zero;
+      Vec8<T> out, gout;
+      out.zero();
+      gout.zero();
       if (ok[u]) {
-        float xf[8], gf[8], yf[8];
-        unpack8(xv[u], xf);
-        unpack8(gv[u], gf);
-        if (MASK) unpack8(yv[u], yf);
+        float xf[8], gf[8];
+        xv[u].get(xf);
+        gv[u].get(gf);
+        pass[u].apply(gf);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if (MASK && !(yf[k] > 0.f)) gf[k] = 0.f;
-          xf[k] = k1[k] * (gf[k] - c1[k] - (xf[k] - m[k]) * c2[k]);
-        }
-        out = pack8(xf);
-        if (dres != nullptr) gout = pack8(gf);
+        for (int k = 0; k < 8; ++k) xf[k] = k1[k] * (gf[k] - c1[k] - (xf[k] - m[k]) * c2[k]);
+        out.set(xf);
+        gout.set(gf);
       }
-      dx[i] = out;
-      if (dres != nullptr) dres[i] = gout;
+      out.store(dx, i);
+      if (dres != nullptr) gout.store(dres, i);
     }
   }
 }
@@ -391,25 +457,110 @@ int reduce_grid(int64_t nvec) {
   int64_t cap = reduce_blocks();
   return (int)(blocks < cap ? (blocks < 1 ? 1 : blocks) : cap);
 }
-bool vector_path(int dtype, int C) {
-  if (dtype != PD_BF16 || (C % 8) != 0) return false;
+// Whole vectors in every row, a power of two of them, and the tensors on 16 bytes.
+bool vector_path(int C, const void* a, const void* b, const void* c, const void* d) {
+  if ((C % 8) != 0) return false;
   const int G = C / 8;
-  return G <= kThreads && (G & (G - 1)) == 0;
+  const uintptr_t all = (uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d;
+  return G <= kThreads && (G & (G - 1)) == 0 && all % 16 == 0;
 }
 int log2i(int v) { int s = 0; while ((1 << s) < v) ++s; return s; }
+
+}  // namespace
+
+namespace {
+
+template <typename T>
+int bn_apply_any(const T* x, const T* res, int64_t rows, int Hp, int Wp, int C, const T* gamma, const T* beta,
+                 const float* mean, const float* invstd, float eps, int relu, T* y, unsigned char* mask, bool vec,
+                 cudaStream_t s) {
+  if (vec) {
+    const int64_t nvec = rows * C / 8;
+    bn_apply_v8_kernel<T><<<vec_grid(nvec, sizeof(T) == 4 ? 2 : 4), kThreads, 0, s>>>(
+        x, res, mean, invstd, eps, gamma, beta, nvec, C / 8, log2i(C / 8), Hp, Wp, relu, y, mask);
+  } else {
+    bn_apply_kernel<T><<<apply_grid(rows * C), kThreads, 0, s>>>(x, res, mean, invstd, eps, gamma, beta, rows, C, Hp, Wp,
+                                                                 relu, y);
+  }
+  PD_LAUNCH_CHECK("bn_apply_kernel");
+  return PD_OK;
+}
+
+template <typename T>
+int bn_fwd_any(const T* x, const T* res, int64_t rows, float count, int Hp, int Wp, int C, const T* gamma, const T* beta,
+               float eps, float momentum, int relu, float* mean, float* invstd, float* running_mean, float* running_var,
+               T* y, unsigned char* mask, float* workspace, bool vec, cudaStream_t s) {
+  const int64_t nvec = rows * C / 8;
+  const int nb = vec ? reduce_grid(nvec * (int)sizeof(T) / 2) : reduce_blocks();
+  if (vec)
+    bn_reduce_v8_kernel<T, 0, 0><<<nb, kThreads, 0, s>>>(x, nullptr, nullptr, nullptr, nullptr, nullptr, nvec, C / 8, C, workspace);
+  else
+    bn_reduce_kernel<T><<<nb, kThreads, 0, s>>>(x, nullptr, nullptr, nullptr, nullptr, rows, C, 0, workspace);
+  PD_LAUNCH_CHECK("bn_reduce_kernel");
+  bn_stats_final_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>(workspace, nb, C, count, eps, momentum, mean, invstd,
+                                                              running_mean, running_var);
+  PD_LAUNCH_CHECK("bn_stats_final_kernel");
+  return bn_apply_any<T>(x, res, rows, Hp, Wp, C, gamma, beta, mean, invstd, -1.f, relu, y, mask, vec, s);
+}
+
+template <typename T, int MASK>
+int bn_bwd_vec(const T* x, const T* dy, const T* y, const unsigned char* mask, int64_t rows, float inv_count, int Hp,
+               int Wp, int C, const T* gamma, const float* mean, const float* invstd, float* dgamma, float* dbeta,
+               int accumulate, T* dx, T* dres, float* sums, float* workspace, cudaStream_t s) {
+  const int64_t nvec = rows * C / 8;
+  const int nb = reduce_grid(nvec * (int)sizeof(T) / 2);
+  bn_reduce_v8_kernel<T, 1, MASK><<<nb, kThreads, 0, s>>>(x, dy, y, mask, mean, invstd, nvec, C / 8, C, workspace);
+  PD_LAUNCH_CHECK("bn_reduce_kernel");
+  bn_bwd_final_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>(workspace, nb, C, sums, dgamma, dbeta, accumulate);
+  PD_LAUNCH_CHECK("bn_bwd_final_kernel");
+  const int grid = vec_grid(nvec, (MASK == 1 || sizeof(T) == 4) ? 2 : 4);
+  bn_bwd_apply_v8_kernel<T, MASK><<<grid, kThreads, 0, s>>>(x, dy, y, mask, mean, invstd, gamma, sums, nvec, C / 8,
+                                                            log2i(C / 8), C, Hp, Wp, inv_count, dx, dres);
+  PD_LAUNCH_CHECK("bn_bwd_apply_kernel");
+  return PD_OK;
+}
+
+template <typename T>
+int bn_bwd_any(const T* x, const T* dy, const T* y, const unsigned char* mask, int64_t rows, float inv_count, int Hp,
+               int Wp, int C, const T* gamma, const float* mean, const float* invstd, float* dgamma, float* dbeta,
+               int accumulate, T* dx, T* dres, float* sums, float* workspace, bool vec, cudaStream_t s) {
+  if (vec && mask != nullptr)
+    return bn_bwd_vec<T, 2>(x, dy, nullptr, mask, rows, inv_count, Hp, Wp, C, gamma, mean, invstd, dgamma, dbeta, accumulate,
+                            dx, dres, sums, workspace, s);
+  if (vec && y != nullptr)
+    return bn_bwd_vec<T, 1>(x, dy, y, nullptr, rows, inv_count, Hp, Wp, C, gamma, mean, invstd, dgamma, dbeta, accumulate, dx,
+                            dres, sums, workspace, s);
+  if (vec)
+    return bn_bwd_vec<T, 0>(x, dy, nullptr, nullptr, rows, inv_count, Hp, Wp, C, gamma, mean, invstd, dgamma, dbeta,
+                            accumulate, dx, dres, sums, workspace, s);
+  const int nb = reduce_blocks();
+  bn_reduce_kernel<T><<<nb, kThreads, 0, s>>>(x, dy, y, mean, invstd, rows, C, 1, workspace);
+  PD_LAUNCH_CHECK("bn_reduce_kernel");
+  bn_bwd_final_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>(workspace, nb, C, sums, dgamma, dbeta, accumulate);
+  PD_LAUNCH_CHECK("bn_bwd_final_kernel");
+  bn_bwd_apply_kernel<T><<<apply_grid(rows * C), kThreads, 0, s>>>(x, dy, y, mean, invstd, gamma, sums, rows, C, Hp, Wp,
+                                                                   inv_count, dx, dres);
+  PD_LAUNCH_CHECK("bn_bwd_apply_kernel");
+  return PD_OK;
+}
 
 }  // namespace
 
 // workspace: fp32 scratch of at least pd_bn_workspace_bytes(C) bytes.
 PD_EXPORT int64_t pd_bn_workspace_bytes(int C) { return (int64_t)reduce_blocks() * 2 * C * sizeof(float); }
 
+// Bytes of the mask that pd_bn_fwd_masked writes for pd_bn_bwd_masked; 0: the shape has none (pass y instead).
+PD_EXPORT int64_t pd_bn_mask_bytes(int N, int H, int W, int C) {
+  return vector_path(C, nullptr, nullptr, nullptr, nullptr) ? (int64_t)N * (H + 2) * (W + 2) * (C / 8) : 0;
+}
+
 // Training forward.  x_pad/y_pad (and res_pad, the optional tensor added before the ReLU): [N,H+2,W+2,C];
 // gamma/beta in `dtype`; mean/invstd: fp32 [C] (out, saved for backward); running_mean/var: fp32 [C],
-// updated in place (may be NULL).
-PD_EXPORT int pd_bn_fwd(int dtype, const void* x_pad, const void* res_pad, int N, int H, int W, int C, const void* gamma,
-                        const void* beta, float eps, float momentum, int relu, float* mean, float* invstd,
-                        float* running_mean, float* running_var, void* y_pad, void* workspace, int64_t workspace_bytes,
-                        void* stream) {
+// updated in place (may be NULL).  mask (may be NULL): pd_bn_mask_bytes bytes, one bit per value (y > 0).
+PD_EXPORT int pd_bn_fwd_masked(int dtype, const void* x_pad, const void* res_pad, int N, int H, int W, int C,
+                               const void* gamma, const void* beta, float eps, float momentum, int relu, float* mean,
+                               float* invstd, float* running_mean, float* running_var, void* y_pad, void* mask,
+                               void* workspace, int64_t workspace_bytes, void* stream) {
   int rc = pd_check_device();
   if (rc != PD_OK) return rc;
   PD_REQUIRE(x_pad && gamma && beta && mean && invstd && y_pad && workspace && N > 0 && H > 0 && W > 0 && C > 0,
@@ -417,84 +568,70 @@ PD_EXPORT int pd_bn_fwd(int dtype, const void* x_pad, const void* res_pad, int N
   PD_REQUIRE(dtype == PD_F32 || dtype == PD_BF16, "pd_bn_fwd: bad dtype");
   PD_REQUIRE(C <= kThreads * kMaxColsPerThread, "pd_bn_fwd: at most %d channels", kThreads * kMaxColsPerThread);
   PD_REQUIRE(workspace_bytes >= pd_bn_workspace_bytes(C), "pd_bn_fwd: workspace too small");
-  cudaStream_t s = (cudaStream_t)stream;
   const int Hp = H + 2, Wp = W + 2;
   const int64_t rows = (int64_t)N * Hp * Wp;
   PD_REQUIRE(rows < (1ll << 31), "pd_bn_fwd: too many rows");
   const float count = (float)((int64_t)N * H * W);
-  const bool vec = vector_path(dtype, C);
-  const int64_t nvec = rows * C / 8;
-  int nb;
-  if (vec) {
-    nb = reduce_grid(nvec);
-    bn_reduce_v8_kernel<0, false><<<nb, kThreads, 0, s>>>((const uint4*)x_pad, nullptr, nullptr, nullptr, nullptr, nvec,
-                                                          C / 8, C, (float*)workspace);
-  } else {
-    nb = reduce_blocks();
-    if (dtype == PD_F32)
-      bn_reduce_kernel<float><<<nb, kThreads, 0, s>>>((const float*)x_pad, nullptr, nullptr, nullptr, nullptr, rows, C, 0, (float*)workspace);
-    else
-      bn_reduce_kernel<__nv_bfloat16><<<nb, kThreads, 0, s>>>((const __nv_bfloat16*)x_pad, nullptr, nullptr, nullptr, nullptr, rows, C, 0, (float*)workspace);
-  }
-  PD_LAUNCH_CHECK("bn_reduce_kernel");
-  bn_stats_final_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)workspace, nb, C, count, eps, momentum,
-                                                              mean, invstd, running_mean, running_var);
-  PD_LAUNCH_CHECK("bn_stats_final_kernel");
-  if (vec) {
-    bn_apply_v8_kernel<<<vec_grid(nvec, 4), kThreads, 0, s>>>((const uint4*)x_pad, (const uint4*)res_pad, mean, invstd,
-                                                               (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta, nvec,
-                                                               C / 8, log2i(C / 8), Hp, Wp, relu, (uint4*)y_pad);
-  } else {
-    const int grid = apply_grid(rows * C);
-    if (dtype == PD_F32)
-      bn_apply_kernel<float><<<grid, kThreads, 0, s>>>((const float*)x_pad, (const float*)res_pad, mean, invstd, (const float*)gamma,
-                                                       (const float*)beta, rows, C, Hp, Wp, relu, (float*)y_pad);
-    else
-      bn_apply_kernel<__nv_bfloat16><<<grid, kThreads, 0, s>>>((const __nv_bfloat16*)x_pad, (const __nv_bfloat16*)res_pad, mean, invstd,
-                                                               (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta, rows, C, Hp, Wp,
-                                                               relu, (__nv_bfloat16*)y_pad);
-  }
-  PD_LAUNCH_CHECK("bn_apply_kernel");
-  return PD_OK;
+  const bool vec = vector_path(C, x_pad, res_pad, y_pad, nullptr);
+  PD_REQUIRE(vec || mask == nullptr, "pd_bn_fwd: no mask for this shape or alignment");
+  if (dtype == PD_F32)
+    return bn_fwd_any<float>((const float*)x_pad, (const float*)res_pad, rows, count, Hp, Wp, C, (const float*)gamma,
+                             (const float*)beta, eps, momentum, relu, mean, invstd, running_mean, running_var, (float*)y_pad,
+                             (unsigned char*)mask, (float*)workspace, vec, (cudaStream_t)stream);
+  using B = __nv_bfloat16;
+  return bn_fwd_any<B>((const B*)x_pad, (const B*)res_pad, rows, count, Hp, Wp, C, (const B*)gamma, (const B*)beta, eps,
+                       momentum, relu, mean, invstd, running_mean, running_var, (B*)y_pad, (unsigned char*)mask,
+                       (float*)workspace, vec, (cudaStream_t)stream);
+}
+
+PD_EXPORT int pd_bn_fwd(int dtype, const void* x_pad, const void* res_pad, int N, int H, int W, int C, const void* gamma,
+                        const void* beta, float eps, float momentum, int relu, float* mean, float* invstd,
+                        float* running_mean, float* running_var, void* y_pad, void* workspace, int64_t workspace_bytes,
+                        void* stream) {
+  return pd_bn_fwd_masked(dtype, x_pad, res_pad, N, H, W, C, gamma, beta, eps, momentum, relu, mean, invstd, running_mean,
+                          running_var, y_pad, nullptr, workspace, workspace_bytes, stream);
+}
+
+static int bn_infer(int dtype, const void* x_pad, const void* res_pad, int N, int H, int W, int C, const void* gamma,
+                    const void* beta, const float* mean, const float* scale, float eps, int relu, void* y_pad, void* stream) {
+  int rc = pd_check_device();
+  if (rc != PD_OK) return rc;
+  PD_REQUIRE(x_pad && gamma && beta && mean && scale && y_pad && N > 0 && H > 0 && W > 0 && C > 0, "pd_bn_apply: bad arguments");
+  PD_REQUIRE(dtype == PD_F32 || dtype == PD_BF16, "pd_bn_apply: bad dtype");
+  const int Hp = H + 2, Wp = W + 2;
+  const int64_t rows = (int64_t)N * Hp * Wp;
+  PD_REQUIRE(rows < (1ll << 31), "pd_bn_apply: too many rows");
+  const bool vec = vector_path(C, x_pad, res_pad, y_pad, nullptr);
+  if (dtype == PD_F32)
+    return bn_apply_any<float>((const float*)x_pad, (const float*)res_pad, rows, Hp, Wp, C, (const float*)gamma,
+                               (const float*)beta, mean, scale, eps, relu, (float*)y_pad, nullptr, vec, (cudaStream_t)stream);
+  using B = __nv_bfloat16;
+  return bn_apply_any<B>((const B*)x_pad, (const B*)res_pad, rows, Hp, Wp, C, (const B*)gamma, (const B*)beta, mean, scale, eps,
+                         relu, (B*)y_pad, nullptr, vec, (cudaStream_t)stream);
 }
 
 // Inference forward: normalises with the given statistics (mean, invstd fp32 [C]).
 PD_EXPORT int pd_bn_apply(int dtype, const void* x_pad, const void* res_pad, int N, int H, int W, int C, const void* gamma,
                           const void* beta, const float* mean, const float* invstd, int relu, void* y_pad, void* stream) {
-  int rc = pd_check_device();
-  if (rc != PD_OK) return rc;
-  PD_REQUIRE(x_pad && gamma && beta && mean && invstd && y_pad && N > 0 && H > 0 && W > 0 && C > 0, "pd_bn_apply: bad arguments");
-  PD_REQUIRE(dtype == PD_F32 || dtype == PD_BF16, "pd_bn_apply: bad dtype");
-  cudaStream_t s = (cudaStream_t)stream;
-  const int Hp = H + 2, Wp = W + 2;
-  const int64_t rows = (int64_t)N * Hp * Wp;
-  PD_REQUIRE(rows < (1ll << 31), "pd_bn_apply: too many rows");
-  if (vector_path(dtype, C)) {
-    const int64_t nvec = rows * C / 8;
-    bn_apply_v8_kernel<<<vec_grid(nvec, 4), kThreads, 0, s>>>((const uint4*)x_pad, (const uint4*)res_pad, mean, invstd,
-                                                               (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta, nvec,
-                                                               C / 8, log2i(C / 8), Hp, Wp, relu, (uint4*)y_pad);
-  } else {
-    const int grid = apply_grid(rows * C);
-    if (dtype == PD_F32)
-      bn_apply_kernel<float><<<grid, kThreads, 0, s>>>((const float*)x_pad, (const float*)res_pad, mean, invstd, (const float*)gamma,
-                                                       (const float*)beta, rows, C, Hp, Wp, relu, (float*)y_pad);
-    else
-      bn_apply_kernel<__nv_bfloat16><<<grid, kThreads, 0, s>>>((const __nv_bfloat16*)x_pad, (const __nv_bfloat16*)res_pad, mean, invstd,
-                                                               (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta, rows, C, Hp, Wp,
-                                                               relu, (__nv_bfloat16*)y_pad);
-  }
-  PD_LAUNCH_CHECK("bn_apply_kernel");
-  return PD_OK;
+  return bn_infer(dtype, x_pad, res_pad, N, H, W, C, gamma, beta, mean, invstd, -1.f, relu, y_pad, stream);
 }
 
-// Training backward.  y_pad != NULL: the forward applied a ReLU and dy is masked by (y > 0) first.
-// dgamma/dbeta: fp32 [C] (stored, or added to when accumulate != 0).  dres_pad (may be NULL): receives
-// the masked dy, i.e. the gradient of the residual input.  sums_ws: fp32 [2*C] scratch.
-PD_EXPORT int pd_bn_bwd(int dtype, const void* x_pad, const void* dy_pad, const void* y_pad, int N, int H, int W, int C,
-                        const void* gamma, const float* mean, const float* invstd, float* dgamma, float* dbeta,
-                        int accumulate, void* dx_pad, void* dres_pad, float* sums_ws, void* workspace,
-                        int64_t workspace_bytes, void* stream) {
+// The same from the running variance (eps >= 0): 1/sqrt(var + eps) is taken in the kernel, which spares the two
+// launches per layer that made up 150 us of a 1.0 ms ResNet-50 forward pass over one image.
+PD_EXPORT int pd_bn_apply_var(int dtype, const void* x_pad, const void* res_pad, int N, int H, int W, int C,
+                              const void* gamma, const void* beta, const float* mean, const float* var, float eps, int relu,
+                              void* y_pad, void* stream) {
+  PD_REQUIRE(eps >= 0.f, "pd_bn_apply_var: eps has to be >= 0");
+  return bn_infer(dtype, x_pad, res_pad, N, H, W, C, gamma, beta, mean, var, eps, relu, y_pad, stream);
+}
+
+// Training backward.  The forward applied a ReLU and dy is masked by (y > 0) first: y_pad != NULL, or mask != NULL (what
+// pd_bn_fwd_masked left, taken instead of y).  dgamma/dbeta: fp32 [C] (stored, or added to when accumulate != 0).
+// dres_pad (may be NULL): receives the masked dy, i.e. the gradient of the residual input.  sums_ws: fp32 [2*C] scratch.
+PD_EXPORT int pd_bn_bwd_masked(int dtype, const void* x_pad, const void* dy_pad, const void* y_pad, const void* mask, int N,
+                               int H, int W, int C, const void* gamma, const float* mean, const float* invstd, float* dgamma,
+                               float* dbeta, int accumulate, void* dx_pad, void* dres_pad, float* sums_ws, void* workspace,
+                               int64_t workspace_bytes, void* stream) {
   int rc = pd_check_device();
   if (rc != PD_OK) return rc;
   PD_REQUIRE(x_pad && dy_pad && gamma && mean && invstd && dx_pad && sums_ws && workspace && N > 0 && H > 0 && W > 0 && C > 0,
@@ -502,55 +639,27 @@ PD_EXPORT int pd_bn_bwd(int dtype, const void* x_pad, const void* dy_pad, const 
   PD_REQUIRE(dtype == PD_F32 || dtype == PD_BF16, "pd_bn_bwd: bad dtype");
   PD_REQUIRE(C <= kThreads * kMaxColsPerThread, "pd_bn_bwd: at most %d channels", kThreads * kMaxColsPerThread);
   PD_REQUIRE(workspace_bytes >= pd_bn_workspace_bytes(C), "pd_bn_bwd: workspace too small");
-  cudaStream_t s = (cudaStream_t)stream;
   const int Hp = H + 2, Wp = W + 2;
   const int64_t rows = (int64_t)N * Hp * Wp;
   PD_REQUIRE(rows < (1ll << 31), "pd_bn_bwd: too many rows");
   const float inv_count = 1.f / (float)((int64_t)N * H * W);
-  const bool vec = vector_path(dtype, C);
-  const int64_t nvec = rows * C / 8;
-  int nb;
-  if (vec) {
-    nb = reduce_grid(nvec);
-    if (y_pad != nullptr)
-      bn_reduce_v8_kernel<1, true><<<nb, kThreads, 0, s>>>((const uint4*)x_pad, (const uint4*)dy_pad, (const uint4*)y_pad, mean,
-                                                           invstd, nvec, C / 8, C, (float*)workspace);
-    else
-      bn_reduce_v8_kernel<1, false><<<nb, kThreads, 0, s>>>((const uint4*)x_pad, (const uint4*)dy_pad, nullptr, mean, invstd, nvec,
-                                                            C / 8, C, (float*)workspace);
-  } else {
-    nb = reduce_blocks();
-    if (dtype == PD_F32)
-      bn_reduce_kernel<float><<<nb, kThreads, 0, s>>>((const float*)x_pad, (const float*)dy_pad, (const float*)y_pad, mean, invstd, rows, C, 1, (float*)workspace);
-    else
-      bn_reduce_kernel<__nv_bfloat16><<<nb, kThreads, 0, s>>>((const __nv_bfloat16*)x_pad, (const __nv_bfloat16*)dy_pad,
-                                                              (const __nv_bfloat16*)y_pad, mean, invstd, rows, C, 1, (float*)workspace);
-  }
-  PD_LAUNCH_CHECK("bn_reduce_kernel");
-  bn_bwd_final_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)workspace, nb, C, sums_ws, dgamma, dbeta, accumulate);
-  PD_LAUNCH_CHECK("bn_bwd_final_kernel");
-  if (vec) {
-    const int grid = vec_grid(nvec, 2);
-    if (y_pad != nullptr)
-      bn_bwd_apply_v8_kernel<true><<<grid, kThreads, 0, s>>>((const uint4*)x_pad, (const uint4*)dy_pad, (const uint4*)y_pad, mean, invstd,
-                                                             (const __nv_bfloat16*)gamma, sums_ws, nvec, C / 8, log2i(C / 8), C, Hp, Wp,
-                                                             inv_count, (uint4*)dx_pad, (uint4*)dres_pad);
-    else
-      bn_bwd_apply_v8_kernel<false><<<grid, kThreads, 0, s>>>((const uint4*)x_pad, (const uint4*)dy_pad, nullptr, mean, invstd,
-                                                              (const __nv_bfloat16*)gamma, sums_ws, nvec, C / 8, log2i(C / 8), C, Hp, Wp,
-                                                              inv_count, (uint4*)dx_pad, (uint4*)dres_pad);
-  } else {
-    const int grid = apply_grid(rows * C);
-    if (dtype == PD_F32)
-      bn_bwd_apply_kernel<float><<<grid, kThreads, 0, s>>>((const float*)x_pad, (const float*)dy_pad, (const float*)y_pad, mean, invstd,
-                                                           (const float*)gamma, sums_ws, rows, C, Hp, Wp, inv_count, (float*)dx_pad,
-                                                           (float*)dres_pad);
-    else
-      bn_bwd_apply_kernel<__nv_bfloat16><<<grid, kThreads, 0, s>>>((const __nv_bfloat16*)x_pad, (const __nv_bfloat16*)dy_pad,
-                                                                   (const __nv_bfloat16*)y_pad, mean, invstd, (const __nv_bfloat16*)gamma,
-                                                                   sums_ws, rows, C, Hp, Wp, inv_count, (__nv_bfloat16*)dx_pad,
-                                                                   (__nv_bfloat16*)dres_pad);
-  }
-  PD_LAUNCH_CHECK("bn_bwd_apply_kernel");
-  return PD_OK;
+  const uintptr_t grads = (uintptr_t)dy_pad | (uintptr_t)dx_pad;
+  const bool vec = vector_path(C, x_pad, (const void*)grads, y_pad, dres_pad);
+  PD_REQUIRE(vec || mask == nullptr, "pd_bn_bwd: no mask for this shape or alignment");
+  if (dtype == PD_F32)
+    return bn_bwd_any<float>((const float*)x_pad, (const float*)dy_pad, (const float*)y_pad, (const unsigned char*)mask, rows,
+                             inv_count, Hp, Wp, C, (const float*)gamma, mean, invstd, dgamma, dbeta, accumulate, (float*)dx_pad,
+                             (float*)dres_pad, sums_ws, (float*)workspace, vec, (cudaStream_t)stream);
+  using B = __nv_bfloat16;
+  return bn_bwd_any<B>((const B*)x_pad, (const B*)dy_pad, (const B*)y_pad, (const unsigned char*)mask, rows, inv_count, Hp, Wp,
+                       C, (const B*)gamma, mean, invstd, dgamma, dbeta, accumulate, (B*)dx_pad, (B*)dres_pad, sums_ws,
+                       (float*)workspace, vec, (cudaStream_t)stream);
+}
+
+PD_EXPORT int pd_bn_bwd(int dtype, const void* x_pad, const void* dy_pad, const void* y_pad, int N, int H, int W, int C,
+                        const void* gamma, const float* mean, const float* invstd, float* dgamma, float* dbeta,
+                        int accumulate, void* dx_pad, void* dres_pad, float* sums_ws, void* workspace,
+                        int64_t workspace_bytes, void* stream) {
+  return pd_bn_bwd_masked(dtype, x_pad, dy_pad, y_pad, nullptr, N, H, W, C, gamma, mean, invstd, dgamma, dbeta, accumulate,
+                          dx_pad, dres_pad, sums_ws, workspace, workspace_bytes, stream);
 }

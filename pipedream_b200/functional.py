@@ -624,16 +624,22 @@ def _bn_ws(device, C):
     return _workspace(device, _lib.load().pd_bn_workspace_bytes(C))
 
 
-def bn_fwd(x_pad, gamma, beta, eps, momentum, relu, running_mean, running_var, res_pad=None):
+def bn_fwd(x_pad, gamma, beta, eps, momentum, relu, running_mean, running_var, res_pad=None, want_mask=False):
+    """(y, mean, invstd), and with want_mask what bn_bwd takes as `mask` in y's place (None where a shape has no mask)."""
     N, Hp, Wp, C = x_pad.shape
     dev = x_pad.device
     mean = torch.empty(C, dtype=torch.float32, device=dev)
     invstd = torch.empty(C, dtype=torch.float32, device=dev)
     y = torch.empty_like(x_pad)
     ws = _bn_ws(dev, C)
-    call("pd_bn_fwd", dt(x_pad), _p(x_pad), _p(res_pad), N, Hp - 2, Wp - 2, C, _p(gamma), _p(beta), float(eps), float(momentum),
-         int(relu), _p(mean), _p(invstd), _p(running_mean), _p(running_var), _p(y), _p(ws), ws.numel(), _stream())
-    return y, mean, invstd
+    mask = None
+    if want_mask and relu and (x_pad.data_ptr() | y.data_ptr() | (res_pad.data_ptr() if res_pad is not None else 0)) % 16 == 0:
+        size = _lib.load().pd_bn_mask_bytes(N, Hp - 2, Wp - 2, C)
+        mask = torch.empty(size, dtype=torch.uint8, device=dev) if size else None
+    call("pd_bn_fwd_masked", dt(x_pad), _p(x_pad), _p(res_pad), N, Hp - 2, Wp - 2, C, _p(gamma), _p(beta), float(eps),
+         float(momentum), int(relu), _p(mean), _p(invstd), _p(running_mean), _p(running_var), _p(y), _p(mask), _p(ws),
+         ws.numel(), _stream())
+    return (y, mean, invstd, mask) if want_mask else (y, mean, invstd)
 
 
 def bn_apply(x_pad, gamma, beta, mean, invstd, relu, res_pad=None):
@@ -644,15 +650,28 @@ def bn_apply(x_pad, gamma, beta, mean, invstd, relu, res_pad=None):
     return y
 
 
-def bn_bwd(x_pad, dy_pad, y_pad, gamma, mean, invstd, dgamma, dbeta, accumulate, want_dres=False):
+def bn_apply_var(x_pad, gamma, beta, mean, var, eps, relu, res_pad=None):
+    """bn_apply from a variance: invstd = rsqrt(var + eps) is taken in the kernel."""
+    if not eps >= 0:                               # the kernel's mark for a finished invstd
+        return bn_apply(x_pad, gamma, beta, mean, torch.rsqrt(var + eps), relu, res_pad)
+    N, Hp, Wp, C = x_pad.shape
+    y = torch.empty_like(x_pad)
+    call("pd_bn_apply_var", dt(x_pad), _p(x_pad), _p(res_pad), N, Hp - 2, Wp - 2, C, _p(gamma), _p(beta), _p(mean), _p(var),
+         float(eps), int(relu), _p(y), _stream())
+    return y
+
+
+def bn_bwd(x_pad, dy_pad, y_pad, gamma, mean, invstd, dgamma, dbeta, accumulate, want_dres=False, mask=None):
     N, Hp, Wp, C = x_pad.shape
     dev = x_pad.device
     dx = torch.empty_like(x_pad)
     dres = torch.empty_like(x_pad) if want_dres else None
     sums = torch.empty(2 * C, dtype=torch.float32, device=dev)
     ws = _bn_ws(dev, C)
-    call("pd_bn_bwd", dt(x_pad), _p(x_pad), _p(dy_pad), _p(y_pad), N, Hp - 2, Wp - 2, C, _p(gamma), _p(mean), _p(invstd),
-         _p(dgamma), _p(dbeta), int(accumulate), _p(dx), _p(dres), _p(sums), _p(ws), ws.numel(), _stream())
+    if dy_pad.data_ptr() % 16 != 0:
+        mask = None
+    call("pd_bn_bwd_masked", dt(x_pad), _p(x_pad), _p(dy_pad), _p(y_pad), _p(mask), N, Hp - 2, Wp - 2, C, _p(gamma), _p(mean),
+         _p(invstd), _p(dgamma), _p(dbeta), int(accumulate), _p(dx), _p(dres), _p(sums), _p(ws), ws.numel(), _stream())
     return (dx, dres) if want_dres else dx
 
 

@@ -228,8 +228,9 @@ class _BatchNormFn(torch.autograd.Function):
         g, b = weight.detach(), bias.detach()
         x_pad = pf.as_padded(x, g.dtype)
         res_pad = pf.as_padded(res, g.dtype) if res is not None else None
-        y_pad, mean, invstd = pf.bn_fwd(x_pad, g, b, mod.eps, mod.momentum if mod.momentum is not None else 0.1,
-                                        fuse_relu, mod.running_mean, mod.running_var, res_pad)
+        y_pad, mean, invstd, ctx.mask = pf.bn_fwd(x_pad, g, b, mod.eps,
+                                                  mod.momentum if mod.momentum is not None else 0.1, fuse_relu,
+                                                  mod.running_mean, mod.running_var, res_pad, want_mask=True)
         ctx.saved = (x_pad, y_pad if fuse_relu else None, mean, invstd)
         ctx.params = (weight, bias)
         ctx.geom = (N, C, H, W)
@@ -249,10 +250,11 @@ class _BatchNormFn(torch.autograd.Function):
         if ctx.has_res and ctx.needs_input_grad[1] and y_pad is not None:
             # the masked upstream gradient is the shortcut's gradient: written by the same pass
             dx_pad, dres_pad = pf.bn_bwd(x_pad, dy_pad, y_pad, g, mean, invstd, grad_buffer(weight), grad_buffer(bias),
-                                         acc, want_dres=True)
+                                         acc, want_dres=True, mask=ctx.mask)
             dres = pf.nchw_view(dres_pad, N, C, H, W)
         else:
-            dx_pad = pf.bn_bwd(x_pad, dy_pad, y_pad, g, mean, invstd, grad_buffer(weight), grad_buffer(bias), acc)
+            dx_pad = pf.bn_bwd(x_pad, dy_pad, y_pad, g, mean, invstd, grad_buffer(weight), grad_buffer(bias), acc,
+                               mask=ctx.mask)
             if ctx.has_res and ctx.needs_input_grad[1]:
                 dres = pf.nchw_view(dy_pad, N, C, H, W)
         return pf.nchw_view(dx_pad, N, C, H, W), dres, None, None, None, None, None
@@ -284,10 +286,9 @@ class NativeBatchNorm2d(nn.Module):
             self.num_batches_tracked.add_(1)
             return _BatchNormFn.apply(x, res, self.weight, self.bias, self, self.fuse_relu, self.out_nchw)
         N, C, H, W = x.shape
-        invstd = torch.rsqrt(self.running_var + self.eps)
-        y_pad = pf.bn_apply(pf.as_padded(x, self.weight.dtype), self.weight.detach(), self.bias.detach(),
-                            self.running_mean, invstd, self.fuse_relu,
-                            pf.as_padded(res, self.weight.dtype) if res is not None else None)
+        y_pad = pf.bn_apply_var(pf.as_padded(x, self.weight.dtype), self.weight.detach(), self.bias.detach(),
+                                self.running_mean, self.running_var, self.eps, self.fuse_relu,
+                                pf.as_padded(res, self.weight.dtype) if res is not None else None)
         return pf.unpack_pnhwc(y_pad) if self.out_nchw else pf.nchw_view(y_pad, N, C, H, W)
 
 

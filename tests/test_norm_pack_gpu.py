@@ -39,3 +39,30 @@ def test_pack_unpack_tiles(shape, src, dst):
         assert torch.equal(pf.pack_pnhwc(s, dst), padded(s, dst))
     pad = padded(x, src)
     assert torch.equal(pf.unpack_pnhwc(pad, dst), x.to(dst))
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=["f32", "bf16"])
+@pytest.mark.parametrize("res", [False, True], ids=["plain", "residual"])
+@pytest.mark.parametrize("shape", [(1, 8, 1, 2), (5, 64, 9, 7), (2, 2048, 3, 3), (9, 256, 28, 28)], ids=str)
+def test_batchnorm_mask(dtype, res, shape):
+    """The mask says y > 0, and the backward pass gives the same from it as from y."""
+    N, C, H, W = shape
+    x, dy = padded(rnd(*shape, seed=3), dtype), padded(rnd(*shape, seed=4), dtype)
+    sc = padded(rnd(*shape, seed=5), dtype) if res else None
+    gamma, beta = (rnd(C, seed=6) * 0.2 + 1).to(dtype), rnd(C, seed=7).to(dtype)
+    y, mean, invstd, mask = pf.bn_fwd(x, gamma, beta, 1e-5, 0.1, True, None, None, sc, want_mask=True)
+    bits = (mask.view(-1, 1) >> torch.arange(8, device="cuda", dtype=torch.uint8)) & 1
+    assert torch.equal(bits.view(y.shape).bool(), y > 0)
+    got = []
+    for kw in ({"mask": mask}, {}):
+        dg, db = torch.empty(C, device="cuda"), torch.empty(C, device="cuda")
+        got.append(pf.bn_bwd(x, dy, y, gamma, mean, invstd, dg, db, False, want_dres=True, **kw) + (dg, db))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
+def test_batchnorm_from_variance():
+    x, gamma, beta = padded(rnd(3, 64, 5, 5, seed=8), torch.bfloat16), rnd(64, seed=9).bfloat16(), rnd(64, seed=10).bfloat16()
+    mean, var = rnd(64, seed=11), rnd(64, seed=12).square()
+    want = pf.bn_apply(x, gamma, beta, mean, torch.rsqrt(var + 1e-5), True)
+    assert torch.equal(pf.bn_apply_var(x, gamma, beta, mean, var, 1e-5, True), want)
