@@ -21,16 +21,25 @@ namespace {
 
 using namespace pd_sm100;
 
-constexpr int kThreads = 192;            // warp 0: TMA producer, warp 1: MMA issuer, warps 2-5: cell epilogue
+constexpr int kMaxStages = 16;
+// warp 0: TMA producer, warp 1: MMA issuer, warps 2-5: cell epilogue, warps 6...: more MMA issuers.  A step is a chain
+// of 64 (backward: 32) small MMAs, and their issue costs more than their work; the K-blocks of a
+// step are dealt out to the issuers, each adds up in columns of its own, and the epilogue adds the parts.
+constexpr int kFwdIssuers = 4;           // one where two CTAs share an SM: more would not leave them the registers
+constexpr int kFwdParts = 4;
+constexpr int kBwdIssuers = 2;
+constexpr int block_threads(int issuers) { return 192 + 32 * (issuers - 1); }
+constexpr int kBwdThreads = block_threads(kBwdIssuers);
 constexpr int kUnits = 8;                // hidden units per CTA
 constexpr int kCols = 4 * kUnits;        // gate columns per CTA = MMA N
 constexpr uint32_t kStageBytes = 128 * kBlockK * 2;      // one [128 x 64] K-block of h: 16 KiB
 constexpr uint32_t kWBlockBytes = kCols * kBlockK * 2;   // one [32 x 64] K-block of the W_hh slice: 4 KiB
 
 struct LstmP {
-  int T, B, H, G, num_stages;
+  int T, B, H, G, num_stages, issuers;
+  int parts;                   // accumulators that a step's K-blocks are dealt out to, whatever the number of issuers
   int Bt, b0;                  // the tensors hold Bt batch rows per time step; this launch works on rows b0 .. b0 + B - 1
-  uint32_t stage_bytes;        // one K-block of the h tile in shared memory: 128 rows (16 KiB), or 64 rows when B <= 64
+  uint32_t stage_bytes;        // one K-block of the h tile in shared memory: B rows rounded up to 8, 128 bytes each
   const __nv_bfloat16* gx;     // [T, B, 4H]
   const __nv_bfloat16* b_hh;   // [4H] or null
   __nv_bfloat16* y;            // [T, B, H]
@@ -65,13 +74,10 @@ __device__ __forceinline__ bool wait_counter(const unsigned int* counter, unsign
 }
 
 // Publish after a named barrier of the 128 epilogue threads: their global writes are ordered before the barrier,
-// one thread then makes them visible device-wide and counts this CTA in (the pattern of a cooperative grid sync).
+// one thread then counts this CTA in with release semantics, which cover what it has observed through the barrier.
 __device__ __forceinline__ void publish_step(unsigned int* counter, bool elected) {
   asm volatile("bar.sync 1, 128;" ::: "memory");
-  if (elected) {
-    __threadfence();
-    atomicAdd(counter, 1u);
-  }
+  if (elected) asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(counter), "r"(1u) : "memory");
 }
 
 // mbarrier wait that also gives up when another role or CTA has reported an error
@@ -88,6 +94,10 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, int* err
       return false;
     }
   }
+}
+
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, int* err, int code) {
+  return __all_sync(0xffffffffu, (int)wait_bar(bar, parity, err, code)) != 0;
 }
 
 __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
@@ -107,23 +117,24 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
   return u;
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+template <int NI>                        // issuer warps (p.issuers of them have work)
+__global__ void __launch_bounds__(block_threads(NI), 1)
 lstm_fwd_persistent_kernel(const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_w,
                            const LstmP p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[8];
-  __shared__ __align__(8) uint64_t empty_bar[8];
+  __shared__ __align__(8) uint64_t full_bar[kMaxStages];
+  __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
   __shared__ __align__(8) uint64_t w_bar;
   __shared__ __align__(8) uint64_t acc_bar;
   __shared__ uint32_t tmem_base_holder;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int S = p.num_stages;
   const int kblocks = p.H / kBlockK;
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_w = smem0;                                        // kblocks x 4 KiB
-  const uint32_t smem_a = smem0 + (uint32_t)kblocks * kWBlockBytes;     // S x 16 KiB (a multiple of 1024 in)
+  const uint32_t smem_a = smem0 + (uint32_t)kblocks * kWBlockBytes;     // S stages (a multiple of 1024 in)
   const int u0 = blockIdx.x * kUnits;
 
   if (threadIdx.x == 0) {
@@ -132,13 +143,13 @@ lstm_fwd_persistent_kernel(const __grid_constant__ CUtensorMap map_h, const __gr
       mbar_init(smem_u32(&empty_bar[s]), 1);
     }
     mbar_init(smem_u32(&w_bar), 1);
-    mbar_init(smem_u32(&acc_bar), 1);
+    mbar_init(smem_u32(&acc_bar), (uint32_t)p.issuers);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(smem_u32(&tmem_base_holder)), "r"(32u) : "memory");
+                 ::"r"(smem_u32(&tmem_base_holder)), "r"((uint32_t)(kFwdParts * kCols)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -173,36 +184,38 @@ lstm_fwd_persistent_kernel(const __grid_constant__ CUtensorMap map_h, const __gr
         }
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------- MMA issuer -------------------------------
-    if (lane == 0) {
-      bool ok = wait_bar(smem_u32(&w_bar), 0, p.err, 6);
-      // The issuing thread runs every instruction between two MMAs itself and an N = 32 MMA is only 16 cycles of
-      // tensor-pipe work, so descriptors advance by 32-bit adds on their low words and the ring position is
-      // carried along instead of being derived by division.
+  } else if (warp == 1 || warp > 5) {
+    // ------------------------------- MMA issuers ------------------------------
+    const int me = warp == 1 ? 0 : warp - 5;
+    if (me < p.issuers) {
+      bool ok = wait_bar_warp(smem_u32(&w_bar), 0, p.err, 6);
+      // (the whole warp walks the loop, see umma_lo_elect)  Descriptors advance by 32-bit adds on
+      // their low words and the ring position is carried along instead of being derived by division.
       const uint64_t da0 = make_desc(smem_a, 0), db0 = make_desc(smem_w, 0);
       const uint32_t a_hi = (uint32_t)(da0 >> 32), b_hi = (uint32_t)(db0 >> 32);
       const uint32_t a_lo0 = (uint32_t)da0, b_lo0 = (uint32_t)db0;
       const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
-      const uint32_t idesc = p.idesc;
-      int s = 0;
-      uint32_t ph = 0, a_lo = a_lo0, fb = full0, eb = empty0;
+      const uint32_t idesc = p.idesc, a_step = p.stage_bytes >> 4;
+      const int issuers = p.issuers;
       for (int t = 1; t < p.T && ok; ++t) {
-        uint32_t b_lo = b_lo0;
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (!wait_bar(fb, ph, p.err, 2)) { ok = false; break; }
+        const uint32_t it0 = (uint32_t)(t - 1) * (uint32_t)kblocks + (uint32_t)me;
+        uint32_t s = it0 % (uint32_t)S, ph = (it0 / (uint32_t)S) & 1u;
+        uint32_t b_lo = b_lo0 + (uint32_t)me * (kWBlockBytes >> 4);
+        for (int kb = me; kb < kblocks; kb += issuers) {
+          if (!wait_bar_warp(full0 + 8u * s, ph, p.err, 2)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (kb == 0) umma_lo<1, 0>(tmem_acc, a_lo, a_hi, b_lo, b_hi, idesc, 0u);
-          else umma_lo<1, 1>(tmem_acc, a_lo, a_hi, b_lo, b_hi, idesc, 1u);
+          const uint32_t a_lo = a_lo0 + s * a_step, acc = tmem_acc + (uint32_t)((kb & (p.parts - 1)) * kCols);
+          if (kb < p.parts) umma_lo_elect<1, 0>(acc, a_lo, a_hi, b_lo, b_hi, idesc, 0u);
+          else umma_lo_elect<1, 1>(acc, a_lo, a_hi, b_lo, b_hi, idesc, 1u);
 #pragma unroll
           for (int kk = 1; kk < kBlockK / 16; ++kk)
-            umma_lo<1, 1>(tmem_acc, a_lo + kk * 2, a_hi, b_lo + kk * 2, b_hi, idesc, 1u);
-          umma_commit(eb);
-          b_lo += kWBlockBytes >> 4;
-          ++s; a_lo += p.stage_bytes >> 4; fb += 8; eb += 8;
-          if (s == S) { s = 0; ph ^= 1u; a_lo = a_lo0; fb = full0; eb = empty0; }
+            umma_lo_elect<1, 1>(acc, a_lo + kk * 2, a_hi, b_lo + kk * 2, b_hi, idesc, 1u);
+          umma_commit_elect(empty0 + 8u * s);
+          b_lo += (uint32_t)issuers * (kWBlockBytes >> 4);
+          s += (uint32_t)issuers;
+          if (s >= (uint32_t)S) { s -= (uint32_t)S; ph ^= 1u; }
         }
-        if (ok) umma_commit(smem_u32(&acc_bar));
+        if (ok) umma_commit_elect(smem_u32(&acc_bar));
       }
     }
   } else {
@@ -238,8 +251,16 @@ lstm_fwd_persistent_kernel(const __grid_constant__ CUtensorMap map_h, const __gr
         ok = all_ok != 0;
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        tmem_ld32(tmem_acc + ((uint32_t)(lg * 32) << 16), r);
+        const uint32_t acc = tmem_acc + ((uint32_t)(lg * 32) << 16);
+        tmem_ld32(acc, r);
         tmem_ld_wait();
+        for (int q = 1; q < p.parts; ++q) {
+          uint32_t r2[kCols];
+          tmem_ld32(acc + (uint32_t)(q * kCols), r2);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < kCols; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+        }
       } else {
 #pragma unroll
         for (int j = 0; j < kCols; ++j) r[j] = 0u;
@@ -294,7 +315,7 @@ lstm_fwd_persistent_kernel(const __grid_constant__ CUtensorMap map_h, const __gr
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(32u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"((uint32_t)(kFwdParts * kCols)) : "memory");
   }
 }
 
@@ -303,30 +324,96 @@ lstm_fwd_persistent_kernel(const __grid_constant__ CUtensorMap map_h, const __gr
 // Backward recurrence, whole sequence in one cooperative kernel (bf16, B <= 128, H a power of two in
 // 128..1024: G = (H/128)^2 CTAs).  Two phases per step, separated by a grid-wide counter:
 //   A(t): cell backward.  CTA c owns the U = H/G hidden units from c*U for all rows: dh = dy[t] + dh_acc,
-//         dgates[t] from the saved activations and cell states, dc carried in a scratch array, dh_acc cleared.
+//         dgates[t] from the saved activations and cell states, dh_acc cleared.
 //   B(t): dh_acc += dgates[t] . W_hh.  CTA (ns, ks) contracts the K slice [512 ks, 512 ks + 512) of the 4H gate
 //         columns into the 128 units of slice ns: its [512 x 128] piece of W_hh sits in shared memory for the
 //         whole sequence (MN-major operand, read in place), dgates[t] streams in by TMA, 32 MMAs of
 //         128 x 128 x 16 accumulate in tensor memory and the epilogue adds the tile to dh_acc with red.v4.f32.
 // ------------------------------------------------------------------------------------------------
-constexpr int kBwdStages = 4;
+constexpr int kBwdMaxStages = 8;
+constexpr uint32_t kBwdRing = 64 * 1024;   // stages of dgates: 4 of 128 rows, 8 of 64 rows or fewer
 constexpr int kBwdN = 128;               // units per N slice
 constexpr int kBwdK = 512;               // gate columns per K slice
 constexpr uint32_t kBwdWBytes = kBwdK * kBwdN * 2;       // 128 KiB
 
 struct LstmBwdP {
-  int T, B, H, G, U, NS;
+  int T, B, H, G, NS;
+  int num_stages;
+  uint32_t stage_bytes;         // as in LstmP
   int Bt, b0;                   // as in LstmP
   const __nv_bfloat16* dy;      // [T, B, H]
   const __nv_bfloat16* act;     // [T, B, 4H]
   const float* c_all;           // [T, B, H]
   __nv_bfloat16* dgates;        // [T, B, 4H]
   float* dh_acc;                // [B, H], zeroed before the launch
-  float* dc;                    // [B, H], zeroed before the launch
   unsigned int* counter;        // zeroed before the launch
   int* err;
   uint32_t idesc;
 };
+
+// What a step's cell backward reads for eight units of a row, except dh: nothing here depends on the chain.
+struct CellIn {
+  uint4 dy, a[4];
+  float4 q0, q1;                // c_{t-1}
+};
+__device__ __forceinline__ void load_cell(CellIn& in, const LstmBwdP& p, int t, int b, int u) {
+  const int H = p.H;
+  const int64_t e = ((int64_t)t * p.Bt + p.b0 + b) * H + u;         // [T,Bt,H] element
+  const int64_t e4 = ((int64_t)t * p.Bt + p.b0 + b) * 4 * H + u;    // [T,Bt,4H] element of gate 0
+  in.dy = *reinterpret_cast<const uint4*>(p.dy + e);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) in.a[g] = *reinterpret_cast<const uint4*>(p.act + e4 + (int64_t)g * H);
+  in.q0 = in.q1 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (t > 0) {
+    in.q0 = *reinterpret_cast<const float4*>(p.c_all + e - (int64_t)p.Bt * H);
+    in.q1 = *(reinterpret_cast<const float4*>(p.c_all + e - (int64_t)p.Bt * H) + 1);
+  }
+}
+// The factors that dh and dc are multiplied with.
+struct CellK { float dy[8], dc[8], f[8], ki[8], kf[8], kg[8], ko[8]; };
+__device__ __forceinline__ void cell_factors(CellK& k, const CellIn& in, const float* ct) {
+  float ai[8], ag[8], ao[8];
+  const float cp[8] = {in.q0.x, in.q0.y, in.q0.z, in.q0.w, in.q1.x, in.q1.y, in.q1.z, in.q1.w};
+  unpack8(in.dy, k.dy);
+  unpack8(in.a[0], ai);
+  unpack8(in.a[1], k.f);
+  unpack8(in.a[2], ag);
+  unpack8(in.a[3], ao);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float tc = tanhf(ct[j]);
+    k.dc[j] = ao[j] * (1.f - tc * tc);
+    k.ki[j] = ag[j] * ai[j] * (1.f - ai[j]);
+    k.kf[j] = cp[j] * k.f[j] * (1.f - k.f[j]);
+    k.kg[j] = ai[j] * (1.f - ag[j] * ag[j]);
+    k.ko[j] = tc * ao[j] * (1.f - ao[j]);
+  }
+}
+// dh_acc is read and cleared, the gate gradients go out, dc moves on one step.
+__device__ __forceinline__ void cell_bwd(const CellK& k, const LstmBwdP& p, int t, int b, int u, float* dc) {
+  const int H = p.H;
+  float4* dhp = reinterpret_cast<float4*>(p.dh_acc + (int64_t)b * H + u);
+  const float4 h0 = __ldcg(dhp), h1 = __ldcg(dhp + 1);
+  const float dhv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+  float gi[8], gf[8], gg[8], go[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float dh = k.dy[j] + dhv[j];
+    const float dcj = dh * k.dc[j] + dc[j];
+    dc[j] = dcj * k.f[j];
+    gi[j] = dcj * k.ki[j];
+    gf[j] = dcj * k.kf[j];
+    gg[j] = dcj * k.kg[j];
+    go[j] = dh * k.ko[j];
+  }
+  __nv_bfloat16* gp = p.dgates + ((int64_t)t * p.Bt + p.b0 + b) * 4 * H + u;
+  *reinterpret_cast<uint4*>(gp) = pack8(gi);
+  *reinterpret_cast<uint4*>(gp + H) = pack8(gf);
+  *reinterpret_cast<uint4*>(gp + 2 * (int64_t)H) = pack8(gg);
+  *reinterpret_cast<uint4*>(gp + 3 * (int64_t)H) = pack8(go);
+  dhp[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+  dhp[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
 
 
 // AND of a flag over the 128 epilogue threads (named barrier 2)
@@ -337,37 +424,42 @@ __device__ __forceinline__ bool all_epilogue(bool ok) {
   return r != 0;
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+// UV: groups of eight units that a thread owns (H / G / 8).  It owns the same ones of the same row in every step, so
+// dc stays in registers.  At UV = 2 (H = 1024) a step's activations are loaded during the previous step's contraction
+// and turned into factors before the wait for dh, which leaves two loads and a few multiplications on the chain.
+template <int UV>
+__global__ void __launch_bounds__(kBwdThreads, 1)
 lstm_bwd_persistent_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_w,
                            const LstmBwdP p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[kBwdStages];
-  __shared__ __align__(8) uint64_t empty_bar[kBwdStages];
+  __shared__ __align__(8) uint64_t full_bar[kBwdMaxStages];
+  __shared__ __align__(8) uint64_t empty_bar[kBwdMaxStages];
   __shared__ __align__(8) uint64_t w_bar;
   __shared__ __align__(8) uint64_t acc_bar;
   __shared__ uint32_t tmem_base_holder;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_w = smem0;                       // 8 K-blocks x 2 atoms x 8 KiB
-  const uint32_t smem_a = smem0 + kBwdWBytes;          // kBwdStages x 16 KiB
+  const uint32_t smem_a = smem0 + kBwdWBytes;          // S stages
+  const int S = p.num_stages;
   const int ns = blockIdx.x % p.NS, ks = blockIdx.x / p.NS;
   constexpr int kKb = kBwdK / kBlockK;                 // 8 K-blocks per step
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kBwdStages; ++s) {
+    for (int s = 0; s < S; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 1);
       mbar_init(smem_u32(&empty_bar[s]), 1);
     }
     mbar_init(smem_u32(&w_bar), 1);
-    mbar_init(smem_u32(&acc_bar), 1);
+    mbar_init(smem_u32(&acc_bar), kBwdIssuers);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(smem_u32(&tmem_base_holder)), "r"(128u) : "memory");
+                 ::"r"(smem_u32(&tmem_base_holder)), "r"((uint32_t)(kBwdIssuers * kBwdN)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -390,42 +482,42 @@ lstm_bwd_persistent_kernel(const __grid_constant__ CUtensorMap map_g, const __gr
         if (!wait_counter(p.counter, (unsigned int)p.G * (unsigned int)(2 * i + 1), p.err, 5)) break;
         asm volatile("fence.proxy.async;" ::: "memory");
         for (int kb = 0; kb < kKb; ++kb, ++it) {
-          const int s = (int)(it % (uint32_t)kBwdStages);
-          const uint32_t ph = (it / (uint32_t)kBwdStages) & 1u;
+          const int s = (int)(it % (uint32_t)S);
+          const uint32_t ph = (it / (uint32_t)S) & 1u;
           if (!wait_bar(smem_u32(&empty_bar[s]), ph ^ 1u, p.err, 1)) { ok = false; break; }
           const uint32_t fb = smem_u32(&full_bar[s]);
-          mbar_expect_tx(fb, kStageBytes);
-          tma_load_2d(smem_a + (uint32_t)s * kStageBytes, &map_g, fb, ks * kBwdK + kb * kBlockK, t * p.Bt + p.b0);
+          mbar_expect_tx(fb, p.stage_bytes);
+          tma_load_2d(smem_a + (uint32_t)s * p.stage_bytes, &map_g, fb, ks * kBwdK + kb * kBlockK, t * p.Bt + p.b0);
         }
       }
     }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = wait_bar(smem_u32(&w_bar), 0, p.err, 6);
+  } else if (warp == 1 || warp > 5) {
+    const int me = warp == 1 ? 0 : warp - 5;
+    {
+      bool ok = wait_bar_warp(smem_u32(&w_bar), 0, p.err, 6);
       // lean issue loop: see the forward kernel
       const uint64_t da0 = make_desc(smem_a, 0), db0 = make_desc(smem_w, 1);
       const uint32_t a_hi = (uint32_t)(da0 >> 32), b_hi = (uint32_t)(db0 >> 32);
       const uint32_t a_lo0 = (uint32_t)da0, b_lo0 = (uint32_t)db0;
       const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
-      const uint32_t idesc = p.idesc;
-      int s = 0;
-      uint32_t ph = 0, a_lo = a_lo0, fb = full0, eb = empty0;
+      const uint32_t idesc = p.idesc, acc = tmem_acc + (uint32_t)(me * kBwdN), a_step = p.stage_bytes >> 4;
       for (int i = 0; i + 1 < p.T && ok; ++i) {
-        uint32_t b_lo = b_lo0;
-        for (int kb = 0; kb < kKb; ++kb) {
-          if (!wait_bar(fb, ph, p.err, 2)) { ok = false; break; }
+        const uint32_t it0 = (uint32_t)(i * kKb + me);
+        uint32_t s = it0 % (uint32_t)S, ph = (it0 / (uint32_t)S) & 1u;
+        for (int kb = me; kb < kKb; kb += kBwdIssuers) {
+          if (!wait_bar_warp(full0 + 8u * s, ph, p.err, 2)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (kb == 0) umma_lo<1, 0>(tmem_acc, a_lo, a_hi, b_lo, b_hi, idesc, 0u);
-          else umma_lo<1, 1>(tmem_acc, a_lo, a_hi, b_lo, b_hi, idesc, 1u);
+          const uint32_t a_lo = a_lo0 + s * a_step, b_lo = b_lo0 + (uint32_t)kb * ((2u * kAtomBytes) >> 4);
+          if (kb == me) umma_lo_elect<1, 0>(acc, a_lo, a_hi, b_lo, b_hi, idesc, 0u);
+          else umma_lo_elect<1, 1>(acc, a_lo, a_hi, b_lo, b_hi, idesc, 1u);
 #pragma unroll
           for (int kk = 1; kk < kBlockK / 16; ++kk)
-            umma_lo<1, 1>(tmem_acc, a_lo + kk * 2, a_hi, b_lo + kk * 128, b_hi, idesc, 1u);
-          umma_commit(eb);
-          b_lo += (2u * kAtomBytes) >> 4;
-          ++s; a_lo += kStageBytes >> 4; fb += 8; eb += 8;
-          if (s == kBwdStages) { s = 0; ph ^= 1u; a_lo = a_lo0; fb = full0; eb = empty0; }
+            umma_lo_elect<1, 1>(acc, a_lo + kk * 2, a_hi, b_lo + kk * 128, b_hi, idesc, 1u);
+          umma_commit_elect(empty0 + 8u * s);
+          s += (uint32_t)kBwdIssuers;
+          if (s >= (uint32_t)S) { s -= (uint32_t)S; ph ^= 1u; }
         }
-        if (ok) umma_commit(smem_u32(&acc_bar));
+        if (ok) umma_commit_elect(smem_u32(&acc_bar));
       }
     }
   } else {
@@ -433,10 +525,39 @@ lstm_bwd_persistent_kernel(const __grid_constant__ CUtensorMap map_g, const __gr
     const int b = lg * 32 + lane;
     const bool row = b < p.B;
     const int H = p.H;
-    const int ua = blockIdx.x * p.U;               // first unit of this CTA's phase-A slice
+    const int ua = blockIdx.x * UV * 8;            // first unit of this CTA's phase-A slice
     bool ok = true;
+    float dc[UV][8];
+#pragma unroll
+    for (int v = 0; v < UV; ++v)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dc[v][j] = 0.f;
+    CellIn in[2];
+    float ct[2][8];                                // cell states of the step at hand
+    auto load_ct = [&](float* c, int t, int u) {
+      const float4* cq = reinterpret_cast<const float4*>(p.c_all + ((int64_t)t * p.Bt + p.b0 + b) * H + u);
+      const float4 c0 = cq[0], c1 = cq[1];
+      c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
+    };
+    if (UV == 2 && row) {
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        load_cell(in[v], p, p.T - 1, b, ua + v * 8);
+        load_ct(ct[v], p.T - 1, ua + v * 8);
+      }
+    }
     for (int i = 0; i < p.T && ok; ++i) {
       const int t = p.T - 1 - i;
+      CellK k[2];
+      if (UV == 2 && row) {
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          cell_factors(k[v], in[v], ct[v]);
+          const float4 q0 = in[v].q0, q1 = in[v].q1;
+          ct[v][0] = q0.x; ct[v][1] = q0.y; ct[v][2] = q0.z; ct[v][3] = q0.w;
+          ct[v][4] = q1.x; ct[v][5] = q1.y; ct[v][6] = q1.z; ct[v][7] = q1.w;
+        }
+      }
       // ---- phase A(t): needs every CTA's B(t+1) contribution to dh_acc
       if (i > 0) {
         bool mine = true;
@@ -445,69 +566,36 @@ lstm_bwd_persistent_kernel(const __grid_constant__ CUtensorMap map_g, const __gr
         if (!ok) break;
       }
       if (row) {
-        for (int u = ua; u < ua + p.U; u += 8) {
-          const int64_t e = ((int64_t)t * p.Bt + p.b0 + b) * H + u;         // [T,Bt,H] element
-          const int64_t e4 = ((int64_t)t * p.Bt + p.b0 + b) * 4 * H + u;    // [T,Bt,4H] element of gate 0
-          const int64_t bh = (int64_t)b * H + u;
-          float dyf[8], ai[8], af[8], ag[8], ao[8];
-          unpack8(*reinterpret_cast<const uint4*>(p.dy + e), dyf);
-          unpack8(*reinterpret_cast<const uint4*>(p.act + e4), ai);
-          unpack8(*reinterpret_cast<const uint4*>(p.act + e4 + H), af);
-          unpack8(*reinterpret_cast<const uint4*>(p.act + e4 + 2 * (int64_t)H), ag);
-          unpack8(*reinterpret_cast<const uint4*>(p.act + e4 + 3 * (int64_t)H), ao);
-          const float4 h0 = __ldcg(reinterpret_cast<const float4*>(p.dh_acc + bh));
-          const float4 h1 = __ldcg(reinterpret_cast<const float4*>(p.dh_acc + bh) + 1);
-          const float4 d0 = *reinterpret_cast<const float4*>(p.dc + bh);
-          const float4 d1 = *(reinterpret_cast<const float4*>(p.dc + bh) + 1);
-          const float4 c0 = *reinterpret_cast<const float4*>(p.c_all + e);
-          const float4 c1 = *(reinterpret_cast<const float4*>(p.c_all + e) + 1);
-          float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
-          if (t > 0) {
-            q0 = *reinterpret_cast<const float4*>(p.c_all + e - (int64_t)p.Bt * H);
-            q1 = *(reinterpret_cast<const float4*>(p.c_all + e - (int64_t)p.Bt * H) + 1);
-          }
-          const float dhv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-          const float dcv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-          const float ct[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-          const float cp[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-          float gi[8], gf[8], gg[8], go[8], dcn[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float dh = dyf[j] + dhv[j];
-            const float tc = tanhf(ct[j]);
-            const float dcj = dh * ao[j] * (1.f - tc * tc) + dcv[j];
-            const float d_o = dh * tc;
-            dcn[j] = dcj * af[j];
-            gi[j] = dcj * ag[j] * ai[j] * (1.f - ai[j]);
-            gf[j] = dcj * cp[j] * af[j] * (1.f - af[j]);
-            gg[j] = dcj * ai[j] * (1.f - ag[j] * ag[j]);
-            go[j] = d_o * ao[j] * (1.f - ao[j]);
+        for (int v = 0; v < UV; ++v) {
+          const int u = ua + v * 8;
+          if (UV > 2) {
+            load_cell(in[0], p, t, b, u);
+            load_ct(ct[0], t, u);
+            cell_factors(k[0], in[0], ct[0]);
           }
-          __nv_bfloat16* gp = p.dgates + e4;
-          *reinterpret_cast<uint4*>(gp) = pack8(gi);
-          *reinterpret_cast<uint4*>(gp + H) = pack8(gf);
-          *reinterpret_cast<uint4*>(gp + 2 * (int64_t)H) = pack8(gg);
-          *reinterpret_cast<uint4*>(gp + 3 * (int64_t)H) = pack8(go);
-          float4* dcp = reinterpret_cast<float4*>(p.dc + bh);
-          dcp[0] = make_float4(dcn[0], dcn[1], dcn[2], dcn[3]);
-          dcp[1] = make_float4(dcn[4], dcn[5], dcn[6], dcn[7]);
-          float4* dhp = reinterpret_cast<float4*>(p.dh_acc + bh);
-          dhp[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-          dhp[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+          cell_bwd(k[UV == 2 ? v : 0], p, t, b, u, dc[v]);
         }
       }
       publish_step(p.counter, warp == 2 && lane == 0);
       if (t == 0) break;
+      if (UV == 2 && row) {                        // in flight during the contraction
+#pragma unroll
+        for (int v = 0; v < 2; ++v) load_cell(in[v], p, t - 1, b, ua + v * 8);
+      }
       // ---- phase B(t): add this CTA's tile of dgates[t] . W_hh to dh_acc
       ok = all_epilogue(wait_bar(smem_u32(&acc_bar), (uint32_t)i & 1u, p.err, 3));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
       for (int cc = 0; cc < kBwdN; cc += 32) {
-        uint32_t r[32];
+        uint32_t r[32], r2[32];
         __syncwarp();
         tmem_ld32(tmem_acc + ((uint32_t)(lg * 32) << 16) + (uint32_t)cc, r);
+        tmem_ld32(tmem_acc + ((uint32_t)(lg * 32) << 16) + (uint32_t)(kBwdN + cc), r2);
         tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 32; ++q) r[q] = __float_as_uint(__uint_as_float(r[q]) + __uint_as_float(r2[q]));
         if (row) {
           float* o = p.dh_acc + (int64_t)b * H + ns * kBwdN + cc;
 #pragma unroll
@@ -527,20 +615,14 @@ lstm_bwd_persistent_kernel(const __grid_constant__ CUtensorMap map_g, const __gr
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(128u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"((uint32_t)(kBwdIssuers * kBwdN)) : "memory");
   }
 }
 
-int g_bwd_state[64];
-
-// Grid-barrier counters of the backward kernel: a ring of slots, one per call (a cooperative kernel owns the
-// whole GPU while it runs, so far fewer than 64 calls are ever in flight on one device).
-__device__ unsigned int g_bwd_counters[64];
-unsigned int* g_bwd_counter_base[64];
-unsigned int g_bwd_next[64];
+int g_bwd_state[64][5];   // per device and log2(UV)
 
 std::mutex g_mu;
-int g_state[64];          // per device: 0 unknown, 1 usable, -1 not usable
+int g_state[64][2];       // per device and kernel: 0 unknown, 1 usable, -1 not usable
 
 }  // namespace
 
@@ -552,8 +634,8 @@ int pd_lstm_fwd_persistent(const void* gx, const void* w_hh, const void* b_hh, i
 }
 
 // The same on the batch rows b0 .. b0 + B - 1 of tensors that hold Bt rows per time step.  Two such launches on two
-// streams (the halves of a batch) run side by side: with B <= 64 the h tile is staged 64 rows at a time and a CTA
-// takes half of an SM's shared memory, so both grids are resident at once and each hides the other's waits.
+// streams (the halves of a batch) run side by side: with B <= 64 a CTA takes half of an SM's shared memory, so both
+// grids are resident at once and each hides the other's waits.
 int pd_lstm_fwd_persistent_rows(const void* gx, const void* w_hh, const void* b_hh, int T, int Bt, int b0, int B, int H,
                                 void* y, void* act, float* c_all, unsigned int* counter, cudaStream_t s) {
   if (B > 128 || H % kBlockK != 0 || H % kUnits != 0 || T < 2 || b0 < 0 || b0 + B > Bt) return 1;
@@ -561,34 +643,41 @@ int pd_lstm_fwd_persistent_rows(const void* gx, const void* w_hh, const void* b_
   const int kblocks = H / kBlockK;
   const uint32_t w_bytes = (uint32_t)kblocks * kWBlockBytes;
   if (w_bytes > 96u * 1024u) return 1;
+  // Only the batch's own rows are staged: every CTA reads all of h_{t-1} from L2 each step, which at 128 rows is 33 MB
+  // per step and was what a step at any batch waited for.  An MMA still reads 128 rows from a stage's start: rows beyond
+  // the batch come from the next stages (behind the last one lies slack) and land in accumulator rows that nobody reads.
+  const int rows = (B + 7) & ~7;
+  const uint32_t stage_bytes = (uint32_t)rows * kBlockK * 2;
   const bool half = B <= 64 && B < Bt;       // one of several launches that share the GPU
-  const uint32_t stage_bytes = half ? kStageBytes / 2 : kStageBytes;
-  const uint32_t budget = half ? 96u * 1024u : 200u * 1024u;     // half: two CTAs (105 KiB each with the slack) per SM
+  const uint32_t budget = (half ? 96u : 200u) * 1024u;           // half: two CTAs (105 KiB each at most) per SM
   if (w_bytes + 2 * stage_bytes > budget) return 1;
   int stages = (int)((budget - w_bytes) / stage_bytes);
-  if (stages > 8) stages = 8;
-  if (stages < 2) return 1;
-  // (an MMA reads 128 rows from a stage's start: with 64-row stages the last one needs 8 KiB of slack behind it)
-  const size_t smem = (size_t)w_bytes + (size_t)stages * stage_bytes + (half ? kStageBytes / 2 : 0) + 1024;
+  if (stages > kMaxStages) stages = kMaxStages;
+  const size_t smem = (size_t)w_bytes + (size_t)stages * stage_bytes + (kStageBytes - stage_bytes) + 1024;
+  const void* kernel = half ? (const void*)lstm_fwd_persistent_kernel<1> : (const void*)lstm_fwd_persistent_kernel<kFwdIssuers>;
+  const int threads = block_threads(half ? 1 : kFwdIssuers);
   int dev = 0;
   PD_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return 1;
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_state[dev] == 0) {
+    if (g_state[dev][half] == 0) {
       int coop = 0, per_sm = 0;
       PD_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-      PD_CUDA(cudaFuncSetAttribute(lstm_fwd_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024));
-      PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lstm_fwd_persistent_kernel, kThreads, 200 * 1024));
-      g_state[dev] = (coop && per_sm >= 1) ? 1 : -1;
+      PD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
+      PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 216 * 1024));
+      g_state[dev][half] = (coop && per_sm >= 1) ? 1 : -1;
     }
-    if (g_state[dev] < 0) return 1;
+    if (g_state[dev][half] < 0) return 1;
   }
   if (G > pd_num_sms()) return 1;
 
   LstmP p;
   memset(&p, 0, sizeof(p));
   p.T = T; p.B = B; p.H = H; p.G = G; p.num_stages = stages;
+  p.parts = kblocks >= 4 ? 4 : (kblocks >= 2 ? 2 : 1);
+  p.issuers = half ? 1 : (kblocks < kFwdIssuers ? kblocks : kFwdIssuers);
+  if (p.issuers > stages) p.issuers = stages;
   p.Bt = Bt; p.b0 = b0; p.stage_bytes = stage_bytes;
   p.gx = (const __nv_bfloat16*)gx; p.b_hh = (const __nv_bfloat16*)b_hh;
   p.y = (__nv_bfloat16*)y; p.act = (__nv_bfloat16*)act; p.c_all = c_all; p.counter = counter;
@@ -596,24 +685,25 @@ int pd_lstm_fwd_persistent_rows(const void* gx, const void* w_hh, const void* b_
   int rc = pd_gemm_error_word(&p.err);
   if (rc != PD_OK) return rc;
   CUtensorMap mh, mw;
-  rc = pd_make_map_2d(&mh, y, (int64_t)T * Bt, H, H, kBlockK, half ? 64 : 128);
+  rc = pd_make_map_2d(&mh, y, (int64_t)T * Bt, H, H, kBlockK, rows);
   if (rc != PD_OK) return rc;
   rc = pd_make_map_2d(&mw, w_hh, 4ll * H, H, H, kBlockK, 8);
   if (rc != PD_OK) return rc;
   PD_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned int), s));
   void* args[] = {(void*)&mh, (void*)&mw, (void*)&p};
-  PD_CUDA(cudaLaunchCooperativeKernel((const void*)lstm_fwd_persistent_kernel, dim3((unsigned)G), dim3(kThreads), args, smem, s));
+  PD_CUDA(cudaLaunchCooperativeKernel(kernel, dim3((unsigned)G), dim3((unsigned)threads), args, smem, s));
   return PD_OK;
 }
 
 // Backward recurrence as one cooperative kernel; same return convention as pd_lstm_fwd_persistent.
-// dh_ws and dc_ws: fp32 [B, H] scratch each.
+// dh_ws and dc_ws: fp32 [B, H] scratch each (dc_ws holds the grid counter: like all of a call's scratch it is the
+// call's own, also where the call has been recorded and is replayed beside others).
 int pd_lstm_bwd_persistent(const void* dy, const void* w_hh, const void* act, const float* c_all, int T, int B, int H,
                            void* dgates, float* dh_ws, float* dc_ws, cudaStream_t s) {
   return pd_lstm_bwd_persistent_rows(dy, w_hh, act, c_all, T, B, 0, B, H, dgates, dh_ws, dc_ws, s);
 }
 
-// Batch rows b0 .. b0 + B - 1 of tensors with Bt rows per time step (dh_ws, dc_ws: [B, H] of this launch alone).  The
+// Batch rows b0 .. b0 + B - 1 of tensors with Bt rows per time step (dh_ws, dc_ws: of this launch alone).  The
 // grid is (H / 128)^2 CTAs - 64 at H = 1024 - so the halves of a batch, launched on two streams, run side by side.
 int pd_lstm_bwd_persistent_rows(const void* dy, const void* w_hh, const void* act, const float* c_all, int T, int Bt,
                                 int b0, int B, int H, void* dgates, float* dh_ws, float* dc_ws, cudaStream_t s) {
@@ -621,49 +711,52 @@ int pd_lstm_bwd_persistent_rows(const void* dy, const void* w_hh, const void* ac
   const int NS = H / kBwdN, KS = 4 * H / kBwdK;
   const int G = NS * KS;
   if (H % G != 0 || (H / G) % 8 != 0 || G > pd_num_sms()) return 1;
-  const size_t smem = (size_t)kBwdWBytes + (size_t)kBwdStages * kStageBytes + 1024;
+  const void* kernel = nullptr;
+  int lg = 0;
+  switch (H / G / 8) {
+    case 2: kernel = (const void*)lstm_bwd_persistent_kernel<2>; lg = 1; break;
+    case 4: kernel = (const void*)lstm_bwd_persistent_kernel<4>; lg = 2; break;
+    case 8: kernel = (const void*)lstm_bwd_persistent_kernel<8>; lg = 3; break;
+    case 16: kernel = (const void*)lstm_bwd_persistent_kernel<16>; lg = 4; break;
+    default: return 1;
+  }
+  const int rows = (B + 7) & ~7;                       // see the forward kernel's launch
+  const uint32_t stage_bytes = (uint32_t)rows * kBlockK * 2;
+  int stages = (int)(kBwdRing / stage_bytes);
+  if (stages > kBwdMaxStages) stages = kBwdMaxStages;
+  const size_t smem = (size_t)kBwdWBytes + (size_t)stages * stage_bytes + (kStageBytes - stage_bytes) + 1024;
   int dev = 0;
   PD_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return 1;
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_bwd_state[dev] == 0) {
+    if (g_bwd_state[dev][lg] == 0) {
       int coop = 0, per_sm = 0;
       PD_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-      PD_CUDA(cudaFuncSetAttribute(lstm_bwd_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024));
-      PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lstm_bwd_persistent_kernel, kThreads, smem));
-      g_bwd_state[dev] = (coop && per_sm >= 1) ? 1 : -1;
+      PD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024));
+      PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBwdThreads, 208 * 1024));
+      g_bwd_state[dev][lg] = (coop && per_sm >= 1) ? 1 : -1;
     }
-    if (g_bwd_state[dev] < 0) return 1;
+    if (g_bwd_state[dev][lg] < 0) return 1;
   }
-  unsigned int* counter = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (g_bwd_counter_base[dev] == nullptr) {
-      unsigned int* base = nullptr;
-      PD_CUDA(cudaGetSymbolAddress((void**)&base, g_bwd_counters));
-      g_bwd_counter_base[dev] = base;
-    }
-    counter = g_bwd_counter_base[dev] + (g_bwd_next[dev]++ % 64u);
-  }
+  unsigned int* counter = reinterpret_cast<unsigned int*>(dc_ws);
   LstmBwdP p;
   memset(&p, 0, sizeof(p));
-  p.T = T; p.B = B; p.H = H; p.G = G; p.U = H / G; p.NS = NS;
+  p.T = T; p.B = B; p.H = H; p.G = G; p.NS = NS; p.num_stages = stages; p.stage_bytes = stage_bytes;
   p.Bt = Bt; p.b0 = b0;
   p.dy = (const __nv_bfloat16*)dy; p.act = (const __nv_bfloat16*)act; p.c_all = c_all;
-  p.dgates = (__nv_bfloat16*)dgates; p.dh_acc = dh_ws; p.dc = dc_ws; p.counter = counter;
+  p.dgates = (__nv_bfloat16*)dgates; p.dh_acc = dh_ws; p.counter = counter;
   p.idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(kBwdN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
   int rc = pd_gemm_error_word(&p.err);
   if (rc != PD_OK) return rc;
   CUtensorMap mg, mw;
-  rc = pd_make_map_2d(&mg, dgates, (int64_t)T * Bt, 4ll * H, 4ll * H, kBlockK, 128);
+  rc = pd_make_map_2d(&mg, dgates, (int64_t)T * Bt, 4ll * H, 4ll * H, kBlockK, rows);
   if (rc != PD_OK) return rc;
   rc = pd_make_map_2d(&mw, w_hh, 4ll * H, H, H, 64, kBlockK);
   if (rc != PD_OK) return rc;
   PD_CUDA(cudaMemsetAsync(dh_ws, 0, (size_t)B * H * sizeof(float), s));
-  PD_CUDA(cudaMemsetAsync(dc_ws, 0, (size_t)B * H * sizeof(float), s));
   PD_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned int), s));
   void* args[] = {(void*)&mg, (void*)&mw, (void*)&p};
-  PD_CUDA(cudaLaunchCooperativeKernel((const void*)lstm_bwd_persistent_kernel, dim3((unsigned)G), dim3(kThreads), args, smem, s));
+  PD_CUDA(cudaLaunchCooperativeKernel(kernel, dim3((unsigned)G), dim3(kBwdThreads), args, smem, s));
   return PD_OK;
 }

@@ -43,6 +43,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* er
     }
   }
 }
+// The same for a whole warp that stays together whatever the outcome (its lanes elect one another afterwards).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* err, int code) {
+  return __all_sync(0xffffffffu, (int)mbar_wait(bar, parity, err, code)) != 0;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -104,6 +108,17 @@ __device__ __forceinline__ void umma_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t
   }
 }
 
+// The same from a whole converged warp, which elects the lane that issues: every operand is warp-uniform then and stays
+// in the uniform registers that tcgen05.mma takes it from.
+template <int CG, int ACC>
+__device__ __forceinline__ void umma_lo_elect(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                              uint32_t idesc, uint32_t acc) {
+  if (elect_one_sync()) umma_lo<CG, ACC>(tmem_d, a_lo, a_hi, b_lo, b_hi, idesc, acc);
+}
+__device__ __forceinline__ void umma_commit_elect(uint32_t bar) {
+  if (elect_one_sync()) umma_commit(bar);
+}
+
 // ---- cta_group::2 (a pair of CTAs in one cluster working on one 256-row tile) ------------------------------
 // The pair's MMA is issued by the even-ranked CTA; each CTA supplies its own 128 rows of A and its half of B
 // from its own shared memory and receives its 128 accumulator rows in its own tensor memory.
@@ -150,6 +165,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() {
