@@ -84,6 +84,7 @@ class StageGraphs:
         self.count = 0                 # recordings held
         self.seen = {}                 # key -> passes run launch by launch so far
         self.minibatches = 0
+        self.last_inputs, self.steady = None, 0      # shapes of the minibatch before; minibatches that had the same in a row
         self.activation_bytes = 0
         self.shadow = None
         self.usable = _ENABLED and rt.device.type == "cuda" and rt.num_ranks_in_stage == 1
@@ -196,6 +197,8 @@ class StageGraphs:
         when the pass ran launch by launch."""
         key, opt = self._key(rt, tensors)
         self.minibatches += 1
+        self.steady = self.steady + 1 if key is not None and key[0] == self.last_inputs else 0
+        self.last_inputs = key[0] if key is not None else None
         p = None
         if key is not None:
             have = self.passes.get(key)
@@ -223,8 +226,10 @@ class StageGraphs:
 
     def _worth_recording(self, rt, key):
         # A recording costs about two passes run launch by launch and pays from then on, so a shape has to have come
-        # back, and the pipeline to have filled and drained about once, before one is made.
-        if self.seen.get(key, 0) < 2 or self.minibatches <= min(8, 2 * rt.num_stages):
+        # back, and the pipeline to have filled and drained about once, before one is made.  Where shapes change from
+        # one minibatch to the next (sentences), few come back often enough: twelve recordings of 25 to 130 ms against
+        # passes of 12 ms made such a stage slower, not faster.
+        if self.seen.get(key, 0) < 1 or self.minibatches <= min(8, 2 * rt.num_stages) or self.steady < 2:
             return False
         if self.count >= MAX_PASSES:
             idle = [q for have in self.passes.values() for q in have if not q.busy]
@@ -275,6 +280,11 @@ class StageGraphs:
                 p.graph = torch.cuda.CUDAGraph()
                 p.graph.capture_begin(capture_error_mode="thread_local")
                 try:
+                    # One block for what the pass will keep, which its tensors are then cut from: hundreds of segments
+                    # of their own took most of a recording's time (37 of 50 ms for a GPT minibatch of 2 x 200 tokens).
+                    block = torch.empty(self.activation_bytes + self.activation_bytes // 8 + (32 << 20),
+                                        dtype=torch.uint8, device=self.device)
+                    del block
                     rt._run_forward(out)
                     if self.dropouts:
                         self.offsets_dev.add_(p.steps_dev)

@@ -69,12 +69,12 @@ def test_recorded_passes_equal_launched_passes(kind, monkeypatch):
 
 
 def test_every_batch_shape_has_its_own_recording(monkeypatch):
-    """Evaluation over batches of changing size: each is answered by its own recording, and the output of one pass is
-    still there after the next."""
+    """Evaluation over batches of two sizes: each is recorded once it has come three times in a row, answered by its own
+    recording from then on, and the output of one pass is still there after the next."""
     torch.manual_seed(0)
     pkg = stages.resnet50(1)
     r, _ = pu.make_worker(pkg, None, None, 1, True, None, shapes=({}, {}))
-    sizes = [3, 1, 3, 1, 3, 1, 3, 1]
+    sizes = [3, 1, 3, 1, 3, 3, 3, 1, 1, 1, 3, 1, 3]
     batches = [next(iter(stages.SyntheticImages(b, 1, seed=7 + b))) for b in sizes]
     r.eval(len(batches))
     r.set_loader(batches)
@@ -84,6 +84,6 @@ def test_every_batch_shape_has_its_own_recording(monkeypatch):
             r.run_forward()
             outs.append(r.output)
             r.run_ack()
-    assert r._graphs.count == 2
+            assert r._graphs.count == (len(outs) > 6) + (len(outs) > 9)
     for b, out in zip(sizes, outs):
         assert torch.equal(out, outs[sizes.index(b)])
