@@ -19,7 +19,7 @@
 #define PD_MAX_TAPS 9
 
 struct PdGemm {
-  int dtype;  // PD_BF16 -> tcgen05, PD_F32 -> SIMT
+  int dtype;  // PD_BF16 -> tcgen05, PD_F32 -> pd_gemm_simt.cu
   const void* a; int64_t a_rows, a_cols, lda; int a_major;
   const void* b; int64_t b_rows, b_cols, ldb; int b_major;
   int M, N, K;

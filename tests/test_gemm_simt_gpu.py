@@ -57,3 +57,42 @@ def test_convolution_passes(N, H, Cin, Cout):
     for split in (0, 1):
         pf.conv2d_wgrad(xp, dyp, dw, dw.stride(0), accumulate=False, split_k=split)
         assert ((dw - ref(x, dy)).abs() <= (N * (H + 2) ** 2 + 8) * eps * ref(x.abs(), dy.abs())).all()
+
+
+# the last output tile and the last chunk of 64 k partly filled; operands whose rows are not on 16 bytes
+@pytest.mark.parametrize("M,N,K", [(2051, 1029, 1000), (1920, 1160, 4608), (2048, 1024, 71)])
+@pytest.mark.parametrize("form", ["nt", "nn", "tn"])
+def test_tensor_core_parts_against_float64(form, M, N, K):
+    """Products large enough for the three-part tile.  Bound: a chunk of 64 k rounds (towards zero) at most six times at
+    the size of its sum, the K/64 chunk sums round to nearest once each, and those roundings are independent."""
+    g = torch.Generator().manual_seed(M + K)
+    a, b = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    ref = a.double() @ b.double().t()
+    if form == "nt":
+        out = pf.gemm_nt(a, b)
+    elif form == "nn":
+        out = pf.gemm_nn(a, b.t().contiguous())
+    else:
+        out = torch.zeros(M, N, device="cuda")
+        pf.gemm_tn(a.t().contiguous(), b.t().contiguous(), out)
+    rel = ((out.double() - ref).norm() / ref.norm()).item()
+    assert rel <= 2.0 ** -24 * (6 + (K / 64) ** 0.5), rel
+    assert pf.gemm_poll_error() == 0
+
+
+def test_tensor_core_parts_keep_infinities():
+    """Values whose parts would multiply to NaN (infinities, and what rounds up to one) give what fp32 gives."""
+    g = torch.Generator().manual_seed(5)
+    a, b = torch.randn(1920, 512, generator=g).cuda(), torch.randn(1160, 512, generator=g).cuda()
+    a[3, 7], a[200, 1], b[5, 2], a[900, 500] = float("inf"), -float("inf"), float("nan"), 3.4e38
+    a[1500], b[1100] = 1e-41, 1e-30                      # subnormal inputs and products
+    out, ref = pf.gemm_nt(a, b), a.double() @ b.double().t()
+    want = ref.float()
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.isinf())
+    assert torch.equal(out[out.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    # relative to a row's products, not to their sum; a part below bf16's smallest step (2^-133) is lost whole, which
+    # shows where a row has subnormal values only
+    A, B = a.double().abs(), b.double().abs()
+    bound = 2.0 ** -20 * (A @ B.t()) + 2.0 ** -133 * (A.sum(1, keepdim=True) + B.sum(1))
+    assert ((out.double() - ref).abs() <= bound)[fine].all()
