@@ -315,8 +315,8 @@ def gemm_nt(a, b, bias=None, relu=False, out_dtype=None, pad_hw=None):
     N = b.shape[0]
     out = torch.empty((M, N), dtype=out_dtype or a.dtype, device=a.device)
     hp, wp = pad_hw if pad_hw is not None else (0, 0)
-    if (a.dtype == torch.bfloat16 and M >= 32 and pad_hw is None and out.dtype in (torch.bfloat16, torch.float32)
-            and not _DETERMINISTIC and (_few_tiles(M, N, K) if M > 128 else K >= 4096 and N <= 16384)):
+    if (a.dtype == torch.bfloat16 and 32 <= M <= 128 and pad_hw is None and K >= 4096 and N <= 16384
+            and out.dtype in (torch.bfloat16, torch.float32) and not _DETERMINISTIC):
         # a few output tiles and a long contraction (a Linear layer at a small batch): split along K over all SMs
         ws = torch.empty(M * N, dtype=torch.float32, device=a.device)
         _timed("gemm_nt", 2.0 * M * N * K, lambda: call(
@@ -331,10 +331,12 @@ def gemm_nt(a, b, bias=None, relu=False, out_dtype=None, pad_hw=None):
 
 
 def _few_tiles(M, N, K):
-    """Whether a product with more than 128 rows is cut along K: a long contraction whose 128 x 128 output tiles leave
-    two thirds of the SMs idle.  Narrower tiles occupy them too, but read operands out of L2 so many times over that L2
-    sets the pace (6.2 TB/s).  400 x 1024 outputs, K = 4096 (32 tiles): 26 -> 16 us; 560 x 1024 (40 tiles): 27 -> 18 us;
-    400 x 1024, K = 50304: 254 -> 50 us; 1050 x 1024, K = 4096 (72 tiles): 27 -> 28 us."""
+    """Whether a data gradient of more than 128 rows is cut along K: a long contraction whose 128 x 128 output tiles
+    leave two thirds of the SMs idle.  Narrower tiles occupy them too, but read operands out of L2 so many times over
+    that L2 sets the pace (6.2 TB/s).  400 x 1024 outputs, K = 4096 (32 tiles): 26 -> 19 us; 560 x 1024 (40 tiles): 25 ->
+    18 us; 400 x 1024, K = 50304: 254 -> 50 us; 1050 x 1024, K = 4096 (72 tiles): 26 -> 30 us.  Forward products are not:
+    the order of the additions varies, and a last bit of a 16-bit activation grows to 2e-2 of the gradients over the
+    decoder's 24 layers."""
     return K >= 2048 and -(-M // 128) * -(-N // 128) <= 48
 
 
@@ -362,7 +364,7 @@ _DETERMINISTIC = False
 def set_deterministic(flag):
     """Weight gradients are normally split along their long contraction (the pixels / tokens of the minibatch) over
     several CTAs that add their parts with fp32 atomics, in an order that changes from run to run (last-bit
-    differences), and so are products with few output tiles and a long contraction.  With this switch every weight gradient is computed without the split: bit-identical from run to
+    differences), and so are data gradients with few output tiles.  With this switch every weight gradient is computed without the split: bit-identical from run to
     run, and several times slower for the layers with few output tiles.  Returns the previous setting."""
     global _DETERMINISTIC
     prev, _DETERMINISTIC = _DETERMINISTIC, bool(flag)

@@ -280,11 +280,6 @@ class StageGraphs:
                 p.graph = torch.cuda.CUDAGraph()
                 p.graph.capture_begin(capture_error_mode="thread_local")
                 try:
-                    # One block for what the pass will keep, which its tensors are then cut from: hundreds of segments
-                    # of their own took most of a recording's time (37 of 50 ms for a GPT minibatch of 2 x 200 tokens).
-                    block = torch.empty(self.activation_bytes + self.activation_bytes // 8 + (32 << 20),
-                                        dtype=torch.uint8, device=self.device)
-                    del block
                     rt._run_forward(out)
                     if self.dropouts:
                         self.offsets_dev.add_(p.steps_dev)

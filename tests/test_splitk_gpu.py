@@ -1,4 +1,5 @@
-"""Products with few output tiles and a long contraction, which are cut along K."""
+"""Products with few output tiles and a long contraction, which are cut along K: data gradients, and Linear layers of up to
+128 rows."""
 import pytest
 import torch
 
