@@ -220,8 +220,6 @@ int pd_gemm_nt_splitk(int dtype, const void* a, int64_t lda, const void* b, int6
                       int out_dtype, int64_t ldo, int M, int N, int K, const void* bias,
                       int bias_dtype, int relu, void* workspace, int64_t workspace_bytes,
                       void* stream);
-int pd_gemm_nn_splitk(int dtype, const void* a, int64_t lda, const void* b, int64_t ldb, void* out, int out_dtype,
-                      int64_t ldo, int M, int N, int K, void* workspace, int64_t workspace_bytes, void* stream);
 int pd_gemm_nn(int dtype, const void* a, int64_t lda, const void* b, int64_t ldb, void* out,
                int out_dtype, int64_t ldo, int M, int N, int K, const void* relu_aux,
                int64_t ld_aux, void* stream);

@@ -107,35 +107,6 @@ splitk_finish_kernel(const float* __restrict__ acc, int M, int N, const void* __
     out[m * ldo + n] = pd_from_float<O>(v);
   }
 }
-// The same for eight neighbouring columns per thread: whole 16-byte vectors of everything.
-__global__ void __launch_bounds__(256)
-splitk_finish_v8_kernel(const float4* __restrict__ acc, long long vecs, int row_vecs, const uint4* __restrict__ bias,
-                        int relu, uint4* __restrict__ out, long long ldo_vecs) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= vecs) return;
-  const long long m = i / row_vecs;
-  const int n = (int)(i - m * row_vecs);
-  const float4 a = acc[2 * i], b = acc[2 * i + 1];
-  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  if (bias != nullptr) {
-    const uint4 u = __ldg(bias + n);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 f = __bfloat1622float2(h[k]);
-      v[2 * k] += f.x;
-      v[2 * k + 1] += f.y;
-    }
-  }
-  uint4 o;
-  __nv_bfloat162* w = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (relu) { v[2 * k] = fmaxf(v[2 * k], 0.f); v[2 * k + 1] = fmaxf(v[2 * k + 1], 0.f); }
-    w[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-  }
-  out[m * ldo_vecs + n] = o;
-}
 }  // namespace
 
 // The same product for a short, wide problem - a Linear layer at a batch of 64: [64, 25088] x [4096, 25088]^T has 16
@@ -144,17 +115,18 @@ splitk_finish_v8_kernel(const float4* __restrict__ acc, long long vecs, int row_
 // ReLU and writes `out`.  The order of the additions varies from run to run (last-bit differences).
 PD_EXPORT int64_t pd_gemm_nt_splitk_workspace_bytes(int M, int N) { return (int64_t)M * N * (int64_t)sizeof(float); }
 
-static int gemm_splitk(int dtype, const void* a, int64_t lda, const void* b, int64_t ldb, int b_major, void* out,
-                       int out_dtype, int64_t ldo, int M, int N, int K, const void* bias, int bias_dtype, int relu,
-                       void* workspace, int64_t workspace_bytes, cudaStream_t s) {
-  PD_REQUIRE(a && b && out && workspace, "pd_gemm_splitk: null pointer");
-  PD_REQUIRE(dtype == PD_BF16, "pd_gemm_splitk: bf16 operands only");
-  PD_REQUIRE(out_dtype == PD_BF16 || out_dtype == PD_F32, "pd_gemm_splitk: bad output type");
-  PD_REQUIRE(workspace_bytes >= pd_gemm_nt_splitk_workspace_bytes(M, N), "pd_gemm_splitk: workspace too small");
+PD_EXPORT int pd_gemm_nt_splitk(int dtype, const void* a, int64_t lda, const void* b, int64_t ldb, void* out,
+                                int out_dtype, int64_t ldo, int M, int N, int K, const void* bias,
+                                int bias_dtype, int relu, void* workspace, int64_t workspace_bytes, void* stream) {
+  PD_REQUIRE(a && b && out && workspace, "pd_gemm_nt_splitk: null pointer");
+  PD_REQUIRE(dtype == PD_BF16, "pd_gemm_nt_splitk: bf16 operands only");
+  PD_REQUIRE(out_dtype == PD_BF16 || out_dtype == PD_F32, "pd_gemm_nt_splitk: bad output type");
+  PD_REQUIRE(workspace_bytes >= pd_gemm_nt_splitk_workspace_bytes(M, N), "pd_gemm_nt_splitk: workspace too small");
+  cudaStream_t s = (cudaStream_t)stream;
   PdGemm g; init(g);
   g.dtype = dtype;
   g.a = a; g.a_rows = M; g.a_cols = K; g.lda = lda; g.a_major = 0;
-  g.b = b; g.b_rows = b_major ? K : N; g.b_cols = b_major ? N : K; g.ldb = ldb; g.b_major = b_major;
+  g.b = b; g.b_rows = N; g.b_cols = K; g.ldb = ldb; g.b_major = 0;
   g.M = M; g.N = N; g.K = K;
   g.out = workspace; g.out_dtype = PD_F32; g.ldo = N;
   const int bn = N > 128 ? 256 : (N > 64 ? 128 : 64);
@@ -164,14 +136,6 @@ static int gemm_splitk(int dtype, const void* a, int64_t lda, const void* b, int
   rc = dispatch(g, s);
   if (rc != PD_OK) return rc;
   const long long total = (long long)M * N;
-  const bool vec = N % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)out | (uintptr_t)workspace | (uintptr_t)bias) % 16 == 0 &&
-                   out_dtype == PD_BF16 && (bias == nullptr || bias_dtype == PD_BF16);
-  if (vec) {
-    splitk_finish_v8_kernel<<<(unsigned)((total / 8 + 255) / 256), 256, 0, s>>>(
-        (const float4*)workspace, total / 8, N / 8, (const uint4*)bias, relu, (uint4*)out, ldo / 8);
-    PD_LAUNCH_CHECK("splitk_finish_v8_kernel");
-    return PD_OK;
-  }
   int grid = (int)((total + 255) / 256);
   if (grid > pd_num_sms() * 8) grid = pd_num_sms() * 8;
   if (out_dtype == PD_BF16)
@@ -181,21 +145,6 @@ static int gemm_splitk(int dtype, const void* a, int64_t lda, const void* b, int
     splitk_finish_kernel<float><<<grid, 256, 0, s>>>((const float*)workspace, M, N, bias, bias_dtype, relu, (float*)out, ldo);
   PD_LAUNCH_CHECK("splitk_finish_kernel");
   return PD_OK;
-}
-
-PD_EXPORT int pd_gemm_nt_splitk(int dtype, const void* a, int64_t lda, const void* b, int64_t ldb, void* out,
-                                int out_dtype, int64_t ldo, int M, int N, int K, const void* bias,
-                                int bias_dtype, int relu, void* workspace, int64_t workspace_bytes, void* stream) {
-  return gemm_splitk(dtype, a, lda, b, ldb, 0, out, out_dtype, ldo, M, N, K, bias, bias_dtype, relu, workspace,
-                     workspace_bytes, (cudaStream_t)stream);
-}
-
-// out[M,N] = a[M,K] . b[K,N] the same way (workspace as above).
-PD_EXPORT int pd_gemm_nn_splitk(int dtype, const void* a, int64_t lda, const void* b, int64_t ldb, void* out,
-                                int out_dtype, int64_t ldo, int M, int N, int K, void* workspace,
-                                int64_t workspace_bytes, void* stream) {
-  return gemm_splitk(dtype, a, lda, b, ldb, 1, out, out_dtype, ldo, M, N, K, nullptr, 0, 0, workspace, workspace_bytes,
-                     (cudaStream_t)stream);
 }
 
 // out[M,N] = a[M,K] . b[K,N]; optional mask: out = aux > 0 ? out : 0   -- Linear data gradient

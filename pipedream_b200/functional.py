@@ -330,28 +330,12 @@ def gemm_nt(a, b, bias=None, relu=False, out_dtype=None, pad_hw=None):
     return out
 
 
-def _few_tiles(M, N, K):
-    """Whether a data gradient of more than 128 rows is cut along K: a long contraction whose 128 x 128 output tiles
-    leave two thirds of the SMs idle.  Narrower tiles occupy them too, but read operands out of L2 so many times over
-    that L2 sets the pace (6.2 TB/s).  400 x 1024 outputs, K = 4096 (32 tiles): 26 -> 19 us; 560 x 1024 (40 tiles): 25 ->
-    18 us; 400 x 1024, K = 50304: 254 -> 50 us; 1050 x 1024, K = 4096 (72 tiles): 26 -> 30 us.  Forward products are not:
-    the order of the additions varies, and a last bit of a 16-bit activation grows to 2e-2 of the gradients over the
-    decoder's 24 layers."""
-    return K >= 2048 and -(-M // 128) * -(-N // 128) <= 48
-
-
 def gemm_nn(a, b, relu_aux=None):
     """a[M,K] . b[K,N], optionally masked by (relu_aux > 0)."""
     _cuda(a, b)
     M, K = a.shape
     N = b.shape[1]
     out = torch.empty((M, N), dtype=a.dtype, device=a.device)
-    if a.dtype == torch.bfloat16 and M > 128 and relu_aux is None and not _DETERMINISTIC and _few_tiles(M, N, K):
-        ws = torch.empty(M * N, dtype=torch.float32, device=a.device)
-        _timed("gemm_nn", 2.0 * M * N * K, lambda: call(
-            "pd_gemm_nn_splitk", dt(a), _p(a), a.stride(0), _p(b), b.stride(0), _p(out), _DT[out.dtype], out.stride(0),
-            M, N, K, _p(ws), ws.numel() * 4, _stream()), (M, N, K))
-        return out
     _timed("gemm_nn", 2.0 * M * N * K, lambda: call(
         "pd_gemm_nn", dt(a), _p(a), a.stride(0), _p(b), b.stride(0), _p(out), _DT[out.dtype], out.stride(0), M, N, K,
         _p(relu_aux), relu_aux.stride(0) if relu_aux is not None else 0, _stream()), (M, N, K))
@@ -364,7 +348,7 @@ _DETERMINISTIC = False
 def set_deterministic(flag):
     """Weight gradients are normally split along their long contraction (the pixels / tokens of the minibatch) over
     several CTAs that add their parts with fp32 atomics, in an order that changes from run to run (last-bit
-    differences), and so are data gradients with few output tiles.  With this switch every weight gradient is computed without the split: bit-identical from run to
+    differences).  With this switch every weight gradient is computed without the split: bit-identical from run to
     run, and several times slower for the layers with few output tiles.  Returns the previous setting."""
     global _DETERMINISTIC
     prev, _DETERMINISTIC = _DETERMINISTIC, bool(flag)
