@@ -231,6 +231,10 @@ class StageGraphs:
         # passes of 12 ms made such a stage slower, not faster.
         if self.seen.get(key, 0) < 1 or self.minibatches <= min(8, 2 * rt.num_stages) or self.steady < 2:
             return False
+        # A recording of the 24-layer decoder (1100 launches a pass, two weight slots, two backward passes each) takes 35 to
+        # 170 ms, four to ten times what a minibatch gains from it: only a run that has settled makes one.
+        if len(self.params) > 200 and self.steady < 64:
+            return False
         if self.count >= MAX_PASSES:
             idle = [q for have in self.passes.values() for q in have if not q.busy]
             oldest = min(idle, key=lambda q: q.last_used, default=None)
